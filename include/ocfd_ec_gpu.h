@@ -331,18 +331,18 @@ int ocfd_profile(ocfd_handle* h, int nsteps, double* phase_ms);
 /* Kernel launches queued by one ocfd_advance step (all of them this library's own kernels). */
 int ocfd_launches_per_step(ocfd_handle* h);
 /* Columns per CTA tile (32 or 64) of the LU-SGS wavefront sweeps, and the wavefront kernel version
- * in use (3: inputs staged by element; 4: staged by 32-byte sector, helper warps off the step's
- * phases; 2: one thread per column).  ocfd_create times each tile width with versions 3 and 4 on
- * the new case (a few steps from freestream, before the state is initialised; the result does not
- * depend on the choice) and keeps the fastest; OCFD_LU_TC=32|64 fixes the width, OCFD_LU_V3=1 or
- * OCFD_LU_V4=1 the version, OCFD_NO_AUTOTUNE=1 takes the first candidate (64 columns if fixed,
- * else 32; version 4 unless fixed). */
+ * in use: 5 (the default, on 32-column tiles: every term evaluated once by the producing cell, one
+ * task per warp); 4: inputs staged by 32-byte sector, 3: by element; 2: one thread per column.  Every
+ * version gives the same results.  OCFD_LU_TC=32|64 fixes the width, OCFD_LU_V3 / V4 / V5=1 the
+ * version; with versions 3 and 4 ocfd_create times what the switches leave open on the new case (a
+ * few steps from freestream, before the state is initialised) and keeps the fastest, unless
+ * OCFD_NO_AUTOTUNE=1, which takes version 4 (64 columns if fixed, else 32) where no version is
+ * fixed. */
 int ocfd_lu_tile_width(const ocfd_handle* h);
 int ocfd_lu_kernel_version(const ocfd_handle* h);
 /* 1 when the two LU-SGS sweeps run as one launch: version 4 in which a block's upper sweep starts
  * as soon as its own lower sweep is done, while deeper blocks still run theirs (OCFD_LU_ONE_LAUNCH=1
- * puts it in version 4's place; same results, measured slower than the two launches once tiles are
- * taken longest first within a level).  ocfd_profile then reports the joint time as the lower
+ * selects it; same results, slower than version 5 and than the two launches of version 4).  ocfd_profile then reports the joint time as the lower
  * sweep's and 0 for the upper. */
 int ocfd_lu_one_launch(const ocfd_handle* h);
 

@@ -41,6 +41,8 @@ struct LuArgs {
   int* blkdone;         // k_lusgs_wave4_ul: per block, lower tiles finished
   int* tile_of;         // per block: first tile index, tiles per row (nJ), tiles per column (nK)
   int* err;             // timeout flag
+  long long* edge;      // version 5: the terms that cross tile edges, one word each (lusgs5.cuh)
+  const long long* edge_off;  // version 5: per tile, its first word in edge
   int TJ, TK;
   long long spin_limit;
 };

@@ -1,529 +1,618 @@
-// LU-SGS sweeps, version 5: inputs packed in sweep order, one bulk copy per step.
+// Version 5 of the LU-SGS sweeps: the pipelined wavefront of lusgs.cuh (same tiles, same order of
+// the dependencies) with the flux-difference terms computed on the producing side and every role of
+// a step on its own warps, joined by mbarriers instead of by CTA-wide barriers.
 //
-// The sweeps (du_LU_SGS, sub_LU_SGS.f90:4-129) march every tile of TJ x TK (j,k) columns along i
-// with a skew (column (lj,lk) is at i = t - lj - lk + 1 at step t of the lower sweep), so each
-// step reads one scattered cell per column from every input plane.  Here a pack kernel, run once
-// per residual before the lower sweep, writes those cells in the order the sweep consumes them:
-// one record per (tile, step) holding, for the tile's columns and a one-column ring around them,
-// every input of that step.  The sweep then fetches a whole step with one cp.async.bulk per
-// record into a ring of shared-memory stages, completed on an mbarrier; it has no per-column
-// address arithmetic or staging bookkeeping left.  Geometry (volumes, face normals and areas) is
-// packed once, when the handle is created.
+// What bounds a sweep is the time of one step of a tile: a block's sweep is a chain of about
+// nx + ny + nz of them.  Versions 3 and 4 take 2,000-3,000 cycles a step on B200: the same U + DU,
+// reciprocal density and pressure are evaluated by three direction threads, each of its divisions
+// is a subroutine of ~125 cycles with a branch, and two CTA barriers, sector bookkeeping and the
+// final divisions sit in the chain.  Here
+//   * a cell, once its DU is known, evaluates the three terms
+//       0.5 (F(U+DU) - F(U)).n S + 0.5 w Lc DU + Lv DU        (sub_LU_SGS.f90:38-117, 135-157)
+//     of its downstream faces itself, so U + DU, 1/rho and p exist once per cell, a cell's
+//     neighbours need nothing of it but these terms, and they cross a tile edge as data (below);
+//   * the quotients by one denominator share its reciprocal: r = RN(1/b), q = RN(x r),
+//     q' = RN(q + r RN(x - b q)), the FMA division of Markstein (IBM J. Res. Dev. 34, 1990; Cornea,
+//     Harrison and Tang, "Scientific Computing on Itanium", 2002), correctly rounded, hence the
+//     bits of x / b, without a branch.  Operands near the limits of the format, infinities and NaN
+//     take the plain division.
 //
-// Both sweeps read the same records: the cells of the upper sweep's step t are those of the lower
-// sweep's step nsteps-1-t, and a column's upstream neighbours of the upper sweep (i+1, j+1, k+1)
-// sit in the next record and in the ring's far side.  The lower sweep writes DU* per record
-// (coalesced); the upper sweep bulk-copies it as its right-hand side, overwrites it with the final
-// DU (what its downstream tiles read) and writes the final DU to the cell-ordered DU planes for
-// the update.
+// Warps of a CTA (TC columns per tile, TC = 32 or 64; RW = TC / 32 warps per group):
+//   L (2 RW)    loads every input plane of the tile in blocks of WB steps, two blocks deep: a request
+//               covers 32 / WB columns times WB consecutive i (a step's own cells lie on 32 different
+//               rows, one sector each, and the L1 miss path takes one sector a cycle, 33 cycles a
+//               warp request: 44 of them a step bounded the first form of this kernel).  The copies
+//               (cp.async) land in rows by step, so a step's cells are one conflict-free row.  L also
+//               stores the finished DU of a block, row-wise the same way;
+//   D0, D1, D2  direction d: DU of the column's cell (each of the three evaluates it: cheaper than
+//               a second barrier), then the term of the downstream face in direction d, into the
+//               next step's slot, and the old state's flux of the next step's face; a step is one
+//               straight-line block, so that these chains overlap;
+//   P0, P1      the diagonal, 1/rho and E - kinetic energy of the old state into the ring of slots
+//               (even and odd steps);
+//   E           one warp: the terms that come from the upstream tiles.
+// One named barrier of the D warps per step (the terms of step t before step t + 1 reads them); P
+// and E run up to SLOTS steps ahead through the ring (full / empty mbarriers), L two blocks.
 //
-// Thread roles: one thread per column (TC threads) evaluates the reference expression of its
-// cell, in the same order and precision as versions 2-4 (the bits equal the hyperplane order);
-// one helper warp issues the bulk copies, releases this tile's progress and waits for the
-// upstream tiles (bounded).  One CTA barrier per step: it orders the neighbours' DU of the
-// previous step (shared memory), frees the ring stage of step t-2 for the next copy, and carries
-// the helper's acquire of the upstream tiles' progress to the threads that then load the
-// cross-tile DU (through L2, one step ahead).
+// Cross-tile terms: an edge column's terms are stored to a buffer of this tile (edge_off), one
+// 8-byte word per value and step, and the consuming tile's warp E polls the words themselves: a
+// word holds the sentinel (all ones, a NaN no arithmetic produces) until its value is stored, and E
+// puts the sentinel back after reading it, so the buffer is ready for the next sweep.  No flag, no
+// fence: one store and one L2 read between tiles.  The wait is bounded (L.spin_limit); E then sets
+// the error flag and delivers zeros without waiting until the tile ends.  Deadlock freedom is that
+// of lusgs.cuh: tiles are handed out in topological order to resident CTAs.
+//
+// Measured (B200, ms lower + upper sweep, the best of versions 3 and 4 -> this): config 2 (2.09 M
+// cells, 8 blocks) FP64 0.690 + 0.669 -> 0.513 + 0.505, mixed 0.623 + 0.664 -> 0.436 + 0.437; 64
+// airfoils mixed 0.742 + 0.704 -> 0.472 + 0.442; wing-body (7.8 M cells, SST) mixed 1.62 + 1.65 -> 1.31
+// + 1.31; one 129 x 33 airfoil FP64 0.194 -> 0.115 a sweep, the 129 x 65 x 17 channel 0.33 -> 0.16.  A
+// step takes about 1,300 cycles: the D warps' shared-memory reads (123 of 8 bytes a thread and step, the
+// burst after the barrier) and L's copies share the SM's load path, about 700 cycles a step together,
+// beside a chain of about 400.  Tried on top and slower: step counters with acquire loads in place of the
+// mbarriers (+3 %), DU shared between the D warps by variables with a second barrier (FP64 +15 %, mixed
+// even), 64-column tiles (+60 %), face geometry and state loaded by the D and P warps themselves into
+// registers (+20 to 40 %).
 #pragma once
-#include <stdint.h>
-
 #include "lusgs.cuh"
 
 namespace ocfd {
 
-// record layout (bytes; every section 16-byte aligned) and per-tile record offsets
-struct LuStream {
-  const LuTile* tmy;       // tiles in block order (index = first + J + nJ*K)
-  const long long* rec0;   // first record of each tile (block order); a tile has nrec + 2 records
-  unsigned char* dyn;      // per-step records: U (ring), R = Res, dt, Lc (ring), Lv (ring)
-  unsigned char* geo;      // static records: vol, n (lower faces), S (lower faces), S (upper faces)
-  double* dus;             // DU records: DU* after the lower sweep, DU after the upper
-  int dyn_bytes, geo_bytes, dus_bytes;
-  int E;                   // columns of the ring-extended tile, (TJ+2)(TK+2)
-  int nstage;              // ring stages in shared memory (as many as fit, 4 to 8)
-  int o_U, o_R, o_dt, o_Lc, o_Lv;     // in a dyn record
-  int o_vol, o_n, o_Slo, o_Sup;        // in a geo record
-};
+constexpr int LU5_PACE = 300;  // ns between a loader warp's requests: keeps bursts off the load path (wing-body sweep 1.37 -> 1.31 ms)
+constexpr long long LU5_EMPTY = -1LL;  // the sentinel of an edge word
 
+// ---- division by a shared reciprocal -------------------------------------------------------
+// RN(1/b) for |b| in 2^-511 .. 2^511: a 20-bit seed, one cubic step (relative error below 2^-58), one
+// correction; for a mantissa of all ones, the one the correction can miss, the result is known
+// (freestream densities one unit below 1 meet it)
+__device__ __forceinline__ double rcp_rn(double b) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+  double e = __fma_rn(-b, y, 1.0);
+  e = __fma_rn(e, e, e);
+  y = __fma_rn(y, e, y);
+  e = __fma_rn(-b, y, 1.0);
+  y = __fma_rn(y, e, y);
+  const bool ones = __double2loint(b) == -1 && (__double2hiint(b) & 0xfffff) == 0xfffff;
+  return ones ? __hiloint2double(__double2hiint(y) & 0xfff00000, 1) : y;
+}
+__device__ __forceinline__ float rcp_rn(float b) { return __frcp_rn(b); }
+// RN(x / b) from r = RN(1/b)
+__device__ __forceinline__ double div_by(double x, double b, double r) {
+  const double q = __dmul_rn(x, r);
+  return __fma_rn(__fma_rn(-b, q, x), r, q);
+}
+__device__ __forceinline__ float div_by(float x, float b, float r) {
+  const float q = __fmul_rn(x, r);
+  return __fmaf_rn(__fmaf_rn(-b, q, x), r, q);
+}
+// the exponent word of |x|, and whether operands lie outside the range div_by is exact in
+__device__ __forceinline__ unsigned expo(double x) { return (unsigned)__double2hiint(x) & 0x7fffffffu; }
+__device__ __forceinline__ unsigned expo(float x) { return (unsigned)__float_as_int(x) & 0x7fffffffu; }
+__device__ __forceinline__ bool bad_den(double b) { return expo(b) - 0x20000000u > 0x3fc00000u; }  // |b| in 2^-511 .. 2^509
+__device__ __forceinline__ bool bad_num(unsigned e, double) { return e > 0x5fc00000u; }
+__device__ __forceinline__ bool bad_den(float b) { return expo(b) - 0x20800000u > 0x3e800000u; }   // 2^-62 .. 2^63
+__device__ __forceinline__ bool bad_num(unsigned e, float) { return e > 0x5f000000u; }
 
-__host__ __device__ inline int lu5_align16(int b) { return (b + 15) & ~15; }
+// The expressions of the flux difference.  FP64 rounds every operation, as the reference; the mixed
+// form contracts them exactly as versions 3 and 4 compile (which product of a sum enters the FMA
+// unrounded was found by comparing bits on random states; the compiler may choose otherwise in other
+// code), so that every version of the sweep gives the same bits.
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ double mad2(double a, double b, double c, double d) { return __dadd_rn(__dmul_rn(a, b), __dmul_rn(c, d)); }  // a b + c d
+__device__ __forceinline__ float mad2(float a, float b, float c, float d) { return __fmaf_rn(a, b, __fmul_rn(c, d)); }
+__device__ __forceinline__ double msub(double a, double b, double c) { return __dsub_rn(__dmul_rn(a, b), c); }  // a b - c
+__device__ __forceinline__ float msub(float a, float b, float c) { return __fmaf_rn(a, b, -c); }
+__device__ __forceinline__ double dot3(const double* u, const double* n) { return __dadd_rn(mad2(u[1], n[0], u[2], n[1]), __dmul_rn(u[3], n[2])); }
+__device__ __forceinline__ float dot3(const float* u, const float* n) { return __fmaf_rn(u[3], n[2], mad2(u[1], n[0], u[2], n[1])); }
+__device__ __forceinline__ double sq3(const double* u) { return __dadd_rn(mad2(u[1], u[1], u[2], u[2]), __dmul_rn(u[3], u[3])); }
+__device__ __forceinline__ float sq3(const float* u) { return __fmaf_rn(u[3], u[3], mad2(u[1], u[1], u[2], u[2])); }
 
-// section offsets for precision T, NV variables, TC columns, E ring columns
-template <class T, int NV>
-inline void lu5_layout(LuStream& S, int TC, int E) {
-  int o = 0;
-  S.o_U = o; o = lu5_align16(o + 8 * NV * E);
-  S.o_R = o; o = lu5_align16(o + (int)sizeof(T) * NV * TC);
-  S.o_dt = o; o = lu5_align16(o + (int)sizeof(T) * TC);
-  S.o_Lc = o; o = lu5_align16(o + (int)sizeof(T) * 3 * E);
-  S.o_Lv = o; o = lu5_align16(o + (int)sizeof(T) * 3 * E);
-  S.dyn_bytes = o;
-  o = 0;
-  S.o_vol = o; o = lu5_align16(o + 8 * TC);
-  S.o_n = o; o = lu5_align16(o + (int)sizeof(T) * 9 * TC);
-  S.o_Slo = o; o = lu5_align16(o + (int)sizeof(T) * 3 * TC);
-  S.o_Sup = o; o = lu5_align16(o + (int)sizeof(T) * 3 * TC);
-  S.geo_bytes = o;
-  S.dus_bytes = lu5_align16(8 * NV * TC);
-  S.E = E;
-  // ring depth: as many stages as fit next to the kernel's static arrays in half of the SM's
-  // 228 KB (two CTAs per SM: every tile of a 2 M-cell case resident at once), 4 at the least
-  const int stat = (2 + 3) * NV * TC * 8 + 2 * TC * 8 + 16 + 1024;
-  const int stg = S.dyn_bytes + S.geo_bytes + S.dus_bytes + 16;
-  S.nstage = (233472 / 2 - 1024 - stat) / stg;
-  if (S.nstage > 8) S.nstage = 8;
-  if (S.nstage < 4) S.nstage = 4;
-}
-
-// the cell of ring column (lj, lk) of a tile in stored record s (record r = s - 1 of the lower
-// sweep): i = r - lj - lk + 1; false when it lies outside the block
-__device__ __forceinline__ bool lu5_cell(const BlkD& B, const LuTile& tl, int s, int lj, int lk, int& i, int& j, int& k) {
-  i = s - 1 - lj - lk + 1;
-  j = tl.j0 + lj;
-  k = tl.k0 + lk;
-  return i >= 1 && i <= B.nx - 1 && j >= 1 && j <= B.ny - 1 && k >= 1 && k <= B.nz - 1;
-}
-
-// per-step inputs of every tile in sweep order; grid.y = tile (block order)
-template <class T, int NV>
-__global__ void k_lu_pack_dyn(Arena<T> A, LuStream S, int TJ, int TK) {
-  const int q = blockIdx.y;
-  const LuTile tl = S.tmy[q];
-  const BlkD& B = A.blk[tl.blk];
-  const int nrec = B.nx - 1 + TJ + TK - 2;
-  const int E = S.E, TC = TJ * TK, W = TJ + 2;
-  const long long tb = A.tot_box, tc = A.tot_cell;
-  const long long n = (long long)(nrec + 2) * E;
-  for (long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x; g < n; g += (long long)gridDim.x * blockDim.x) {
-    const int s = (int)(g / E), e = (int)(g - (long long)s * E);
-    const int lj = e % W - 1, lk = e / W - 1;
-    unsigned char* rec = S.dyn + (S.rec0[q] + s) * (long long)S.dyn_bytes;
-    double* U = (double*)(rec + S.o_U);
-    T* Lc = (T*)(rec + S.o_Lc);
-    T* Lv = (T*)(rec + S.o_Lv);
-    int i, j, k;
-    const bool ok = lu5_cell(B, tl, s, lj, lk, i, j, k);
-    const bool core = lj >= 0 && lj < TJ && lk >= 0 && lk < TK;
-    double u[NV];
-    T lc[3], lv[3], r[NV], dt = T(0);
-    if (ok) {
-      const long long bi = bix(B, i, j, k), ci = cix(B, i, j, k);
-#pragma unroll
-      for (int m = 0; m < NV; m++) {
-        const double x = A.U[m * tb + bi];
-        u[m] = m >= 5 ? clamp0(x) : x;   // as limit_vt leaves U6 / U7 (sub_time_advance.f90:410-443)
-      }
-#pragma unroll
-      for (int d = 0; d < 3; d++) { lc[d] = A.Lc[d * tc + ci]; lv[d] = A.Lv[d * tc + ci]; }
-      if (core) {
-#pragma unroll
-        for (int m = 0; m < NV; m++) r[m] = A.Res[m * tc + ci];
-        dt = A.dt[ci];
-      }
-    } else {
-#pragma unroll
-      for (int m = 0; m < NV; m++) { u[m] = 0.0; r[m] = T(0); }
-#pragma unroll
-      for (int d = 0; d < 3; d++) { lc[d] = T(0); lv[d] = T(0); }
-    }
-#pragma unroll
-    for (int m = 0; m < NV; m++) U[m * E + e] = u[m];
-#pragma unroll
-    for (int d = 0; d < 3; d++) { Lc[d * E + e] = lc[d]; Lv[d * E + e] = lv[d]; }
-    if (core) {
-      const int c = lj + TJ * lk;
-      T* R = (T*)(rec + S.o_R);
-#pragma unroll
-      for (int m = 0; m < NV; m++) R[m * TC + c] = r[m];
-      ((T*)(rec + S.o_dt))[c] = dt;
-    }
-  }
-}
-
-// static geometry records (once per handle); grid.y = tile (block order)
-template <class T>
-__global__ void k_lu_pack_geo(Arena<T> A, LuStream S, int TJ, int TK) {
-  const int q = blockIdx.y;
-  const LuTile tl = S.tmy[q];
-  const BlkD& B = A.blk[tl.blk];
-  const int nrec = B.nx - 1 + TJ + TK - 2;
-  const int TC = TJ * TK;
-  const long long tf = A.tot_face;
-  const long long n = (long long)(nrec + 2) * TC;
-  for (long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x; g < n; g += (long long)gridDim.x * blockDim.x) {
-    const int s = (int)(g / TC), c = (int)(g - (long long)s * TC);
-    const int lj = c % TJ, lk = c / TJ;
-    unsigned char* rec = S.geo + (S.rec0[q] + s) * (long long)S.geo_bytes;
-    int i, j, k;
-    const bool ok = lu5_cell(B, tl, s, lj, lk, i, j, k);
-    double vol = 0.0;
-    T nn[9], slo[3], sup[3];
-#pragma unroll
-    for (int x = 0; x < 9; x++) nn[x] = T(0);
-#pragma unroll
-    for (int d = 0; d < 3; d++) { slo[d] = T(0); sup[d] = T(0); }
-    if (ok) {
-      vol = A.vold[cix(B, i, j, k)];
-      const long long f = fix_(B, i, j, k);
-#pragma unroll
-      for (int d = 0; d < 3; d++) {
-        nn[3 * d + 0] = A.M[(M_NI1 + 3 * d) * tf + f];
-        nn[3 * d + 1] = A.M[(M_NI2 + 3 * d) * tf + f];
-        nn[3 * d + 2] = A.M[(M_NI3 + 3 * d) * tf + f];
-        slo[d] = A.M[(M_SI + d) * tf + f];
-        // the upper sweep pairs the lower face's normal with the upper face's area
-        // (sub_LU_SGS.f90:96-97, 105-106, 114-115)
-        sup[d] = A.M[(M_SI + d) * tf + fix_(B, i + (d == 0), j + (d == 1), k + (d == 2))];
-      }
-    }
-    ((double*)(rec + S.o_vol))[c] = vol;
-    T* N = (T*)(rec + S.o_n);
-#pragma unroll
-    for (int x = 0; x < 9; x++) N[x * TC + c] = nn[x];
-#pragma unroll
-    for (int d = 0; d < 3; d++) { ((T*)(rec + S.o_Slo))[d * TC + c] = slo[d]; ((T*)(rec + S.o_Sup))[d * TC + c] = sup[d]; }
-  }
-}
-
-// ---- mbarrier + bulk copy (sm_90+ PTX; no multicast) --------------------------------------
-__device__ __forceinline__ unsigned lu5_s(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void lu5_mbar_init(uint64_t* bar, unsigned count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(lu5_s(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void lu5_mbar_fence_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
-__device__ __forceinline__ void lu5_mbar_expect(uint64_t* bar, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(lu5_s(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void lu5_bulk(void* dst, const void* src, unsigned bytes, uint64_t* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-               ::"r"(lu5_s(dst)), "l"(src), "r"(bytes), "r"(lu5_s(bar)) : "memory");
-}
-__device__ __forceinline__ bool lu5_mbar_test(uint64_t* bar, unsigned parity) {
+// ---- mbarriers -----------------------------------------------------------------------------
+__device__ __forceinline__ void mb_init(unsigned a, int n) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(a), "r"(n) : "memory"); }
+__device__ __forceinline__ bool mb_try(unsigned a, unsigned parity) {
   unsigned ok;
-  asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-               : "=r"(ok) : "r"(lu5_s(bar)), "r"(parity) : "memory");
+  asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(ok) : "r"(a), "r"(parity) : "memory");
   return ok != 0;
 }
-// bounded wait for the phase of the given parity; false on timeout
-__device__ __forceinline__ bool lu5_mbar_wait(uint64_t* bar, unsigned parity, long long limit) {
-  long long it = 0;
-  while (!lu5_mbar_test(bar, parity)) {
-    if (++it > limit) return false;
-  }
-  return true;
+__device__ __forceinline__ void mb_arrive(unsigned a) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(a) : "memory"); }
+// waits for the phase of the given parity; bounded (another role of the CTA always makes progress:
+// the bound only turns a defect into an error)
+__device__ __forceinline__ void mb_wait(unsigned a, unsigned parity, int* err) {
+  for (int n = 0; !mb_try(a, parity);)
+    if (++n > 20000000) { atomicExch(err, 1); return; }
 }
-
-// barrier 1 of the compute groups alone (warp-uniform callers; barrier 0 is __syncthreads)
-template <int NT>
-__device__ __forceinline__ void lu5_bar_compute() { asm volatile("bar.sync 1, %0;" ::"n"(NT) : "memory"); }
-
-template <class T, int NV, bool UPPER>
-__host__ __device__ inline int lu5_stage_bytes(const LuStream& S) { return S.dyn_bytes + S.geo_bytes + (UPPER ? S.dus_bytes : 0); }
-
-template <class T, int NV, int TC>
-inline size_t lu5_smem(const LuStream& S, bool upper) {
-  return (size_t)S.nstage * (S.dyn_bytes + S.geo_bytes + (upper ? S.dus_bytes : 0)) + 16 * S.nstage;
+__device__ __forceinline__ long long ld_word(const long long* p) {
+  long long v;
+  asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
 }
-// shared memory of the kernel outside the ring (DU exchange, direction terms, diagonal, tile id)
-template <int NV, int TC>
-constexpr size_t lu5_static_smem() { return (2 + 3) * NV * TC * 8 + 2 * TC * 8 + 16; }
+__device__ __forceinline__ void st_word(long long* p, long long v) { asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(v) : "memory"); }
 
-// Thread groups of a CTA (TC threads each, one per column): 0, 1, 2 the direction threads (the
-// flux-difference term of the upstream neighbour in i, j, k; its old-state half is prepared a
-// step ahead, so only the DU-dependent half sits on the dependency chain), 3 the owner (the
-// diagonal, and the final sum and division of the variables 3..NV-1; direction thread d finishes
-// variable d), then one helper warp.  Two CTA barriers per step: B1 (the previous step's DU is in
-// shared memory; a ring stage is free), B2 (the three terms and the diagonal are in shared memory).
+// one element of at most 8 bytes into shared memory, and this thread's copies onto an mbarrier
+template <class X>
+__device__ __forceinline__ void cp_elem(unsigned dst, const X* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst), "l"(src), "n"((int)sizeof(X)) : "memory");
+}
+__device__ __forceinline__ void cp_arrive(unsigned a) { asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(a) : "memory"); }
+
+// ---- shared memory (byte offsets) -------------------------------------------------------------
+// Input rows: one row of TC cells per stream and step, 2 WB rows per stream (two blocks).  The row
+// pitch is TC + 2 doubles or TC + 4 floats: the copies of a request (32 / WB columns x WB steps, a
+// column's step being its i plus its skew) then fall into different banks.
+// The right-hand side's rows hold doubles in every form: DU overwrites them.
+// Slots (one per step, SLOTS of them): the terms of the three directions for the step's cells, a
+// row of TC own columns followed by TC places for the upstream edges (placed so that a warp's read
+// of own and edge columns is free of bank conflicts), and what P computes.
 template <class T, int NV, bool UPPER, int TC>
-__global__ void __launch_bounds__(4 * TC + 32, 2) k_lusgs_wave5(Arena<T> A, LuArgs L, LuStream S) {
-  extern __shared__ __align__(128) unsigned char s_dyn[];
-  __shared__ double s_du[2][NV][TC];     // DU of each column's cell of the last two steps
-  __shared__ double s_acc[3][NV][TC];    // the direction terms of the current step
-  __shared__ double s_diag[2][TC];       // the diagonal: every variable's, the SA variable's
+struct Lu5Smem {
+  using RT = typename std::conditional<UPPER, double, T>::type;  // right-hand side: Res (lower) or DU* (upper)
+  static constexpr int WB = TC == 64 ? 4 : 8, ROWS = 2 * WB, SLOTS = TC == 64 ? 3 : 4;
+  static constexpr int PB = (TC + 2) * 8, PT = sizeof(T) == 8 ? PB : (TC + 4) * 4;
+  static constexpr int U = 0, R = U + NV * ROWS * PB, VOL = R + NV * ROWS * PB, DT = VOL + ROWS * PB;
+  static constexpr int LC = DT + ROWS * PT, LV = LC + 3 * ROWS * PT, N = LV + 3 * ROWS * PT, S = N + 9 * ROWS * PT;
+  static constexpr int SLOT0 = S + 3 * ROWS * PT;
+  static constexpr int NA = sizeof(T) == 8 ? (NV == 6 ? 4 : 2) : (NV == 6 ? 2 : 1);  // diagonal: (value and) reciprocal, SA's own
+  static constexpr int AS = 2 * TC + 2;  // the place behind the edges stays zero
+  static constexpr int ACC = 0, AL = ACC + 3 * NV * AS * 8, Q = AL + NA * TC * 8;  // Q: 1/rho, E - kinetic energy
+  static constexpr int SU = Q + 2 * TC * (int)sizeof(T);                         // mixed form: the state in FP32
+  static constexpr int SLOT = (SU + (sizeof(T) == 4 ? NV * TC * 4 : 0) + 15) / 16 * 16;
+  static constexpr int BYTES = SLOT0 + SLOTS * SLOT;
+  static_assert(SLOT0 % 16 == 0 && BYTES <= 227 * 1024, "shared memory of one CTA");
+};
+template <class T, int NV, bool UPPER, int TC>
+inline size_t lu5_smem() { return (size_t)Lu5Smem<T, NV, UPPER, TC>::BYTES; }
+template <int TC>
+constexpr int lu5_threads() { return 7 * TC + 32; }
+
+template <class T, int NV, bool UPPER, int TC>
+__global__ void __launch_bounds__(7 * TC + 32, 1) k_lusgs_wave5(Arena<T> A, LuArgs L) {
+  using SM = Lu5Smem<T, NV, UPPER, TC>;
+  using RT = typename SM::RT;
+  constexpr int SLOTS = SM::SLOTS, WB = SM::WB, RW = TC / 32, NA = SM::NA, PB = SM::PB, PT = SM::PT, ROWS = SM::ROWS;
+  constexpr bool FP64 = sizeof(T) == 8;
+  constexpr int AS5 = NV == 6 ? 2 : 0;  // the SA variable's own diagonal (FP64 form: value, reciprocal)
+  extern __shared__ __align__(16) unsigned char s_dyn[];
+  __shared__ __align__(8) unsigned long long s_bar[3 * SLOTS + 4];
   __shared__ int s_tile;
-  const int NS = S.nstage;
-  const int stage_bytes = lu5_stage_bytes<T, NV, UPPER>(S);
-  uint64_t* bars = (uint64_t*)(s_dyn + (size_t)NS * stage_bytes);
-  auto stage = [&](long long seq) { return s_dyn + (size_t)(seq % NS) * stage_bytes; };
-  auto wait_rec = [&](long long seq) { return lu5_mbar_wait(bars + seq % NS, (unsigned)((seq / NS) & 1), L.spin_limit); };
-  const int tid = threadIdx.x;
-  const int grp = tid < 4 * TC ? tid / TC : 4;
-  const int TJ = L.TJ, TK = L.TK, E = S.E, W = TJ + 2;
-  const int c = tid % TC, lj = c % TJ, lk = c / TJ;
-  const int ec = (lj + 1) + W * (lk + 1);   // this column in the ring-extended tile
-  const int HT = 4 * TC;                     // the helper thread
-  constexpr bool MIXED = sizeof(T) == 4;     // the mixed form (FP32 fluxes, FP64 state / diagonal)
-  const long long tc = A.tot_cell;
-  if (tid == HT) {
-    for (int q = 0; q < NS; q++) lu5_mbar_init(bars + q, 1);
-    lu5_mbar_fence_init();
+  const long long tb = A.tot_box, tf = A.tot_face, tc = A.tot_cell;
+  const int TJ = L.TJ, TK = L.TK;
+  const int tid = threadIdx.x, role = tid / TC, c = tid % TC, lane = tid & 31;  // roles 0..2: D, 3, 4: P, 5, 6: L, 7: E
+  const int lj = c % TJ, lk = c / TJ;
+  if (TJ * TK != TC || TK < 2 || TJ < 4 || TJ + TK > TC / 2 + 2) {  // a tile shape the edge and bank layouts do not cover: refuse
+    if (tid == 0) atomicExch(L.err, 1);
+    return;
   }
-  __syncthreads();
-  long long seq0 = 0;   // records this CTA has loaded before the current tile
+  // full (P's values), full (upstream terms), empty barrier of each slot; full and empty of the two row blocks
+  const unsigned fullP = (unsigned)__cvta_generic_to_shared(s_bar), fullE = fullP + 8 * SLOTS, empty0 = fullP + 16 * SLOTS;
+  const unsigned fullR = fullP + 24 * SLOTS, emptyR = fullR + 16;
+  if (tid == 0) {
+    for (int q = 0; q < SLOTS; q++) { mb_init(fullP + 8 * q, RW); mb_init(fullE + 8 * q, 1); mb_init(empty0 + 8 * q, 3 * RW); }
+    for (int q = 0; q < 2; q++) { mb_init(fullR + 8 * q, 2 * TC); mb_init(emptyR + 8 * q, 3 * RW); }
+  }
+  for (int q = tid; q < SLOTS * 3 * NV; q += lu5_threads<TC>())  // the zero places
+    reinterpret_cast<double*>(s_dyn + SM::SLOT0 + q / (3 * NV) * SM::SLOT + SM::ACC)[(q % (3 * NV)) * SM::AS + 2 * TC] = 0.0;
+  // steps and row blocks this CTA has done (the same in every role): slot it % SLOTS, round
+  // it / SLOTS; block buffer ib % 2, round ib / 2
+  unsigned it = 0, ib = 0;
   for (;;) {
+    __syncthreads();
     if (tid == 0) s_tile = atomicAdd(&L.counter[UPPER ? 1 : 0], 1);
     __syncthreads();
-    const int qq = s_tile;
-    if (qq >= L.ntiles) break;
-    const LuTile tl = UPPER ? L.rtiles[qq] : L.tiles[qq];
+    const int q = s_tile;
+    if (q >= L.ntiles) break;
+    const LuTile tl = UPPER ? L.rtiles[q] : L.tiles[q];
     const BlkD& B = A.blk[tl.blk];
-    const SolveP& sp = A.sp[B.solve];
+    const SolveP& s = A.sp[B.solve];
     const int nxm = B.nx - 1, nym = B.ny - 1, nzm = B.nz - 1;
+    const int j = UPPER ? (tl.j0 + TJ - 1 - lj) : (tl.j0 + lj);
+    const int k = UPPER ? (tl.k0 + TK - 1 - lk) : (tl.k0 + lk);
+    const bool active = j >= 1 && j <= nym && k >= 1 && k <= nzm;
     const int* tb3 = L.tile_of + 3 * tl.blk;
     const int first = tb3[0], nJ = tb3[1], nK = tb3[2];
     const int J = (tl.j0 - 1) / TJ, K = (tl.k0 - 1) / TK;
-    const int my = first + J + nJ * K;
-    int pj = -1, pk = -1;   // upstream tiles (block order)
-    if (!UPPER) {
-      if (J > 0) pj = my - 1;
-      if (K > 0) pk = my - nJ;
-    } else {
-      if (J < nJ - 1) pj = my + 1;
-      if (K < nK - 1) pk = my + nJ;
-    }
-    const int nsteps = nxm + TJ + TK - 2;
-    const int nrecs = nsteps + 2;
-    const long long r0 = S.rec0[my];
-    // the x-th record loaded is stored record x (lower) or nrecs-1-x (upper); step t's own
-    // record is load t+1, its neighbours' record load t (the previous step's own one)
-    auto rec_of_load = [&](int x) { return UPPER ? (nrecs - 1 - x) : x; };
-    const double w = sp.w_lu, gamma = sp.gamma;
-    const bool visc = sp.viscous == 1;
-    const bool dual = sp.time_method == -1;
-    const double sfac1 = dual ? A.sfac[1] : 0.0;
-    const int j = tl.j0 + lj, k = tl.k0 + lk;
-    const bool active = j <= nym && k <= nzm;
-    auto own_s = [&](int t) { return UPPER ? (nsteps - t) : (t + 1); };
-    auto cell_i = [&](int t) { return own_s(t) - lj - lk; };
-    auto on_at = [&](int t) { const int i = cell_i(t); return active && t < nsteps && i >= 1 && i <= nxm; };
-    auto has = [&](int d, int i) {
-      return UPPER ? (d == 0 ? i != nxm : (d == 1 ? j != nym : k != nzm)) : (d == 0 ? i != 1 : (d == 1 ? j != 1 : k != 1));
-    };
-    // the final value of variable m at step t (sub_LU_SGS.f90:65-67 lower, 120-122 upper).  The
-    // FP64 form divides by the diagonal as the reference does; the mixed form multiplies by its
-    // FP64 reciprocal, taken by the owner off the dependency chain
-    auto finish = [&](int m, int t) {
-      const unsigned char* so = stage(seq0 + t + 1);
-      const double dg = (NV == 6 && m == 5) ? s_diag[1][c] : s_diag[0][c];
-      double r;
-      if (!UPPER) {
-        const double x = (double)((const T*)(so + S.o_R))[m * TC + c] + s_acc[0][m][c] + s_acc[1][m][c] + s_acc[2][m][c];
-        r = MIXED ? x * dg : x / dg;
-      } else {
-        const double x = s_acc[0][m][c] + s_acc[1][m][c] + s_acc[2][m][c];
-        r = ((const double*)(so + S.dyn_bytes + S.geo_bytes))[m * TC + c] + (MIXED ? x * dg : x / dg);
-      }
-      return r;
-    };
-    auto store = [&](int m, int t, double r) {
-      s_du[t & 1][m][c] = r;
-      S.dus[(r0 + own_s(t)) * (S.dus_bytes / 8) + m * TC + c] = r;
-      if (UPPER) A.DU[m * tc + cix(B, cell_i(t), j, k)] = r;
-    };
-
-    if (grp == 4) {
-      // ---- helper: bulk copies, progress release, upstream waits ----------------------
-      auto issue = [&](int x) {
-        if (x < 0 || x >= nrecs) return;
-        const long long seq = seq0 + x;
-        unsigned char* st = stage(seq);
-        uint64_t* bar = bars + seq % NS;
-        const long long rs = r0 + rec_of_load(x);
-        lu5_mbar_expect(bar, (unsigned)stage_bytes);
-        lu5_bulk(st, S.dyn + rs * S.dyn_bytes, S.dyn_bytes, bar);
-        lu5_bulk(st + S.dyn_bytes, S.geo + rs * S.geo_bytes, S.geo_bytes, bar);
-        if (UPPER) lu5_bulk(st + S.dyn_bytes + S.geo_bytes, (const unsigned char*)S.dus + rs * S.dus_bytes, S.dus_bytes, bar);
+    const int nsteps = nxm + TJ + TK - 2, nblk = (nsteps + WB - 1) / WB;
+    auto on_at = [&](int t) { const int il = t - lj - lk; return active && il >= 0 && il < nxm; };
+    auto slot_of = [&](unsigned n) { return s_dyn + SM::SLOT0 + (n % SLOTS) * SM::SLOT; };
+    auto row_of = [&](int t) { return (int)((ib + t / WB) & 1) * WB + t % WB; };  // the row of step t in every stream
+    if (role < 3) {
+      // ------------------------------------------------------------------ direction warps
+      const int d = role;
+      const double w = s.w_lu;
+      const bool visc = NV >= 6 || s.viscous == 1;  // a turbulence model implies the viscous terms
+      const T g1 = (T)(s.gamma - 1.0), half = (T)0.5;
+      const bool has_j = UPPER ? j != nym : j != 1, has_k = UPPER ? k != nzm : k != 1;  // upstream neighbours
+      // places of the upstream terms: the own column's, its neighbours' (or the upstream edges' behind
+      // them), or the zero place where there is no neighbour
+      const int a_i = c * 8, a_z = 2 * TC * 8;
+      const int a_j = (NV * SM::AS + (!has_j ? 2 * TC : (lj > 0 ? c - 1 : TC + c + TJ - 1))) * 8;
+      const int a_k = (2 * NV * SM::AS + (!has_k ? 2 * TC : (lk > 0 ? c - TJ : TC + TC - TJ + lj))) * 8;
+      // does this column's term leave the tile?  Edge words: j edge [step][m][lk], then k edge [step][m][lj]
+      const bool out = d == 1 ? (lj == TJ - 1 && (UPPER ? J > 0 : J < nJ - 1)) : (d == 2 && lk == TK - 1 && (UPPER ? K > 0 : K < nK - 1));
+      const int ow = d == 1 ? TK : TJ;
+      long long* const eout = L.edge + L.edge_off[first + J + nJ * K] + (d == 1 ? lk : (long long)nsteps * NV * TK + lj);
+      struct Cell {
+        T U[NV], r0, ei, g[6];  // state, 1/rho, E - kinetic energy; downstream face: normal, area / 2; w Lc / 2, Lv
+        RT R[NV];
+        double al[NA];
       };
-      int seen_j = 0, seen_k = 0;
-      auto poll = [&](int t) {   // the upstream tiles have done the steps whose DU step t reads
-        if (t >= nsteps) return;
-        bool ok = true;
-        if (pj >= 0 && seen_j < min(t + TJ, nsteps)) ok &= wait_ge(L.progress + pj, min(t + TJ, nsteps), L.spin_limit, seen_j);
-        if (pk >= 0 && seen_k < min(t + TK, nsteps)) ok &= wait_ge(L.progress + pk, min(t + TK, nsteps), L.spin_limit, seen_k);
-        if (!ok) atomicExch(L.err, 1);
-      };
-      if (tid == HT) {
-        for (int x = 0; x < NS - 1; x++) issue(x);
-        poll(0);
-        poll(1);
-      }
-      __syncthreads();   // B0
-      for (int t = 0; t < nsteps; t++) {
-        __syncthreads();   // B1 (the compute groups' B2 is a named barrier without the helper, so
-                           // the release fence and the upstream wait below overlap their step)
-        if (tid == HT) {
-          if (t > 0) st_release(L.progress + my, t);
-          issue(t + NS - 1);   // into the stage of load t-1, last read before B1
-          poll(t + 2);
+      auto take = [&](Cell& x, const unsigned char* sl, int row) {
+        const unsigned char* const r8 = s_dyn + row * PB + c * 8;
+        const unsigned char* const rt = s_dyn + row * PT + c * (int)sizeof(T);
+#pragma unroll
+        for (int m = 0; m < NV; m++) {
+          if (FP64) {
+            const double u = *reinterpret_cast<const double*>(r8 + SM::U + m * ROWS * PB);
+            x.U[m] = (T)(m >= 5 ? clamp0(u) : u);
+          } else {
+            x.U[m] = reinterpret_cast<const T*>(sl + SM::SU)[m * TC + c];
+          }
+          x.R[m] = *reinterpret_cast<const RT*>(s_dyn + SM::R + (m * ROWS + row) * PB + c * (int)sizeof(RT));
         }
-      }
-    } else if (grp == 3) {
-      // ---- owner: diagonal (sub_LU_SGS.f90:29-39, 82-92), finish of variables 3..NV-1 ----
-      __syncthreads();   // B0
-      for (int t = 0; t < nsteps; t++) {
-        __syncthreads();   // B1
-        const bool on = on_at(t);
-        if (on) {
-          if (!wait_rec(seq0 + t + 1)) atomicExch(L.err, 1);
-          const unsigned char* so = stage(seq0 + t + 1);
-          const T* Lco = (const T*)(so + S.o_Lc);
-          const T* Lvo = (const T*)(so + S.o_Lv);
-          const double vol = ((const double*)(so + S.dyn_bytes + S.o_vol))[c];
-          const double dt = (double)((const T*)(so + S.o_dt))[c];
-          const double a0 = vol / dt + w * ((double)Lco[ec] + (double)Lco[E + ec] + (double)Lco[2 * E + ec]);
-          double al = a0, als = a0;
-          if (visc) {
-            const double lv0 = Lvo[ec], lv1 = Lvo[E + ec], lv2 = Lvo[2 * E + ec];
-            const double lv = lv0 + lv1 + lv2;
-            al = al + 2.0 * lv;
-            als = als + 2.0 * lv;
-            if (NV == 6) {
-              if (!UPPER) als = als + lv;
-              else als = als + lv0 + lv1 + lv2;
+#pragma unroll
+        for (int m = 0; m < 3; m++) x.g[m] = *reinterpret_cast<const T*>(rt + SM::N + (3 * d + m) * ROWS * PT);
+        // halving is exact: 0.5 (DF S + w Lc DU) = DF (S / 2) + (w Lc / 2) DU in every rounding
+        x.g[3] = (T)(UPPER ? -0.5 : 0.5) * *reinterpret_cast<const T*>(rt + SM::S + d * ROWS * PT);
+        x.g[4] = (T)0.5 * (T)(w * (double)*reinterpret_cast<const T*>(rt + SM::LC + d * ROWS * PT));
+        x.g[5] = *reinterpret_cast<const T*>(rt + SM::LV + d * ROWS * PT);
+#pragma unroll
+        for (int m = 0; m < NA; m++) x.al[m] = reinterpret_cast<const double*>(sl + SM::AL)[m * TC + c];
+        x.r0 = reinterpret_cast<const T*>(sl + SM::Q)[c];
+        x.ei = reinterpret_cast<const T*>(sl + SM::Q)[TC + c];
+      };
+      // F(U).n of the old state (plain: by plain division); true: operands div_by does not cover
+      auto old_flux = [&](const Cell& x, T* F, bool plain) -> bool {
+        const T dot = dot3(x.U, x.g);
+        const T un = plain ? dot / x.U[0] : div_by(dot, x.U[0], x.r0);
+        const T p = mul_rn(g1, x.ei);
+        F[0] = x.U[0] * un;
+#pragma unroll
+        for (int m = 1; m < 4; m++) F[m] = NV == 7 && m == 3 ? mad2(p, x.g[2], x.U[3], un) : mad2(x.U[m], un, p, x.g[m - 1]);
+        F[4] = add_rn(x.U[4], p) * un;
+#pragma unroll
+        for (int m = 5; m < NV; m++) F[m] = x.U[m] * un;
+        return bad_den(x.U[0]) || bad_num(expo(dot), dot);
+      };
+      // DU of the cell (sub_LU_SGS.f90:63-72 lower, 108-117 upper) from the sum xs, and the term v of
+      // its downstream face; plain and the result as above
+      auto cell = [&](const Cell& x, const T* F, const double* xs, double* DU, double* v, bool plain) -> bool {
+        unsigned e = 0;
+#pragma unroll
+        for (int m = 0; m < NV; m++) {
+          if (FP64) {
+            const int q5 = m == 5 ? AS5 : 0;
+            DU[m] = plain ? xs[m] / x.al[q5] : div_by(xs[m], x.al[q5], x.al[q5 + 1]);
+            if (UPPER) DU[m] = (double)x.R[m] + DU[m];
+            e = max(e, expo(xs[m]));
+          } else {  // the mixed form multiplies by the diagonal's FP64 reciprocal
+            const double ra = x.al[NV == 6 && m == 5 ? 1 : 0];
+            DU[m] = UPPER ? __fma_rn(xs[m], ra, (double)x.R[m]) : __dmul_rn(xs[m], ra);
+          }
+        }
+        bool bad = FP64 && (bad_num(e, 0.0) || bad_den(x.al[0]) || bad_den(x.al[AS5 < NA ? AS5 : 0]));
+        T U2[NV];
+#pragma unroll
+        for (int m = 0; m < NV; m++) U2[m] = (T)__dadd_rn((double)x.U[m], DU[m]);  // DU rounded first, in the mixed form too
+        const T r2 = rcp_rn(U2[0]);
+        const T dot = dot3(U2, x.g), kin = half * sq3(U2);
+        const T un = plain ? dot / U2[0] : div_by(dot, U2[0], r2);
+        const T ke = plain ? kin / U2[0] : div_by(kin, U2[0], r2);
+        bad = bad || bad_den(U2[0]) || bad_num(max(expo(dot), expo(kin)), dot);
+        const T p = mul_rn(g1, U2[4] - ke);
+        T DF[NV];
+        DF[0] = msub(U2[0], un, F[0]);
+#pragma unroll
+        for (int m = 1; m < 4; m++) DF[m] = (m == 3 || (NV == 7 && m == 2) ? mad2(p, x.g[m - 1], U2[m], un) : mad2(U2[m], un, p, x.g[m - 1])) - F[m];
+        DF[4] = msub(add_rn(U2[4], p), un, F[4]);
+#pragma unroll
+        for (int m = 5; m < NV; m++) DF[m] = msub(U2[m], un, F[m]);
+#pragma unroll
+        for (int m = 0; m < NV; m++) {
+          if (!FP64) {  // off-diagonal products in FP32, the sum stays FP64
+            const float du = (float)DU[m], y = __fmaf_rn((float)DF[m], (float)x.g[3], __fmul_rn((float)x.g[4], du));
+            v[m] = (double)(visc ? __fmaf_rn((float)x.g[5], du, y) : y);
+          } else {
+            const double y = mad2((double)DF[m], (double)x.g[3], (double)x.g[4], DU[m]);
+            v[m] = visc ? y + (double)x.g[5] * DU[m] : y;
+          }
+        }
+        return bad;
+      };
+      T F[2][NV];
+      Cell x[2];
+      mb_wait(fullP + 8 * (it % SLOTS), (it / SLOTS) & 1, L.err);
+      take(x[0], slot_of(it), row_of(0));
+      if (old_flux(x[0], F[0], false)) old_flux(x[0], F[0], true);
+      for (int t0 = 0; t0 < nsteps; t0 += 2) {
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+          const int t = t0 + u;
+          if (t >= nsteps) break;
+          const unsigned n = it + t;
+          const unsigned char* const sl = slot_of(n);
+          unsigned char* const ns = slot_of(n + 1);
+          Cell& xc = x[u];
+          Cell& xn = x[1 - u];
+          // the upstream terms of this step and P's values of the next one (there is none after the
+          // last); P has read its inputs from the rows of that step, so D may
+          {
+            const unsigned ea = fullE + 8 * (n % SLOTS), ep = (n / SLOTS) & 1;
+            const unsigned pa = t + 1 < nsteps ? fullP + 8 * ((n + 1) % SLOTS) : ea, pp = t + 1 < nsteps ? ((n + 1) / SLOTS) & 1 : ep;
+            const bool e0 = mb_try(ea, ep), p0 = mb_try(pa, pp);
+            if (!(e0 && p0)) { mb_wait(ea, ep, L.err); mb_wait(pa, pp, L.err); }
+          }
+          cta_bar_id<1, 3 * TC>();  // the terms of step t - 1 are in slot t
+          double xs[NV];
+          {
+            const unsigned char* const acc = sl + SM::ACC;
+            const int ai = t - lj - lk > 0 ? a_i : a_z;
+#pragma unroll
+            for (int m = 0; m < NV; m++) {
+              const double a0 = *reinterpret_cast<const double*>(acc + ai + m * SM::AS * 8);
+              const double a1 = *reinterpret_cast<const double*>(acc + a_j + m * SM::AS * 8);
+              const double a2 = *reinterpret_cast<const double*>(acc + a_k + m * SM::AS * 8);
+              xs[m] = UPPER ? a0 + a1 + a2 : (double)xc.R[m] + a0 + a1 + a2;
             }
           }
-          if (dual) {
-            al = al + sfac1 * vol;
-            als = als + sfac1 * vol;
+          take(xn, ns, row_of(t + 1));
+          const bool on = on_at(t);
+          double DU[NV], v[NV];
+          const bool bad = cell(xc, F[u], xs, DU, v, false);
+          const bool badn = old_flux(xn, F[1 - u], false);
+          if ((bad && on) || badn) {
+            cell(xc, F[u], xs, DU, v, true);
+            old_flux(xn, F[1 - u], true);
           }
-          s_diag[0][c] = MIXED ? 1.0 / al : al;
-          s_diag[1][c] = MIXED ? 1.0 / als : als;
-        }
-        lu5_bar_compute<4 * TC>();   // B2
-        if (on) {
-          double r[NV];
+          double* const nacc = reinterpret_cast<double*>(ns + SM::ACC) + d * NV * SM::AS + c;
 #pragma unroll
-          for (int m = 3; m < NV; m++) r[m] = finish(m, t);
+          for (int m = 0; m < NV; m++) nacc[m * SM::AS] = v[m];
+          if (out && on) {
 #pragma unroll
-          for (int m = 3; m < NV; m++) store(m, t, r[m]);
+            for (int m = 0; m < NV; m++) st_word(eout + t * (NV * ow) + m * ow, __double_as_longlong(v[m]));
+          }
+          if (d == 0) {  // over the right-hand side's row of this step
+            double* const o = reinterpret_cast<double*>(s_dyn + SM::R + row_of(t) * PB) + c;
+#pragma unroll
+            for (int m = 0; m < NV; m++) o[m * ROWS * (PB / 8)] = DU[m];
+          }
+          __syncwarp();
+          if (lane == 0) {
+            mb_arrive(empty0 + 8 * (n % SLOTS));  // this warp's reads of slot t are done
+            if (t % WB == WB - 1 || t == nsteps - 1) mb_arrive(emptyR + 8 * ((ib + t / WB) & 1));  // and the block's
+          }
         }
       }
-    } else {
-      // ---- direction thread d --------------------------------------------------------
-      const int d = grp;
-      const int dnb = UPPER ? 1 : -1;
-      const int en = d == 0 ? ec : (d == 1 ? ec + dnb : ec + dnb * W);       // the neighbour's ring column
-      const int cn = d == 0 ? c : (d == 1 ? c + dnb : c + dnb * TJ);          // ... and its column (in-tile)
-      // a neighbour in another tile: its DU comes through L2 after the helper's wait.  Lower j-1 of
-      // column (0, lk) is column (TJ-1, lk) of tile J-1, TJ-1 records later (the skew); upper j+1
-      // of column (TJ-1, lk) is column (0, lk) of tile J+1, TJ-1 records earlier; likewise in k
-      const bool xt = d == 1 ? (UPPER ? (lj == TJ - 1 && pj >= 0) : (lj == 0 && pj >= 0))
-                             : (d == 2 ? (UPPER ? (lk == TK - 1 && pk >= 0) : (lk == 0 && pk >= 0)) : false);
-      const long long pr0 = !xt ? 0 : S.rec0[d == 1 ? pj : pk];
-      const int colp = d == 1 ? (UPPER ? TJ * lk : (TJ - 1 + TJ * lk)) : (UPPER ? lj : (lj + TJ * (TK - 1)));
-      const int dsp = d == 1 ? (UPPER ? -(TJ - 1) : (TJ - 1)) : (UPPER ? -(TK - 1) : (TK - 1));
-      auto load_x = [&](int t, double* xd) {
-        const double* src = S.dus + (pr0 + own_s(t) + dsp) * (S.dus_bytes / 8) + colp;
+    } else if (role < 5) {
+      // ------------------------------------------------------------------ diagonal and old-state values
+      const double w = s.w_lu;
+      const bool visc = NV >= 6 || s.viscous == 1, dual = s.time_method == -1;
+      const double sfac1 = dual ? A.sfac[1] : 0.0;
+      const T half = (T)0.5;
+      for (int t = role - 3; t < nsteps; t += 2) {  // even or odd steps of the tile
+        const unsigned n = it + t, rb = ib + t / WB;
+        unsigned char* const sl = slot_of(n);
+        if (t % WB < 2) mb_wait(fullR + 8 * (rb & 1), (rb >> 1) & 1, L.err);  // this warp's first step of the block
+        const int row = row_of(t);
+        const unsigned char* const r8 = s_dyn + row * PB + c * 8;
+        const unsigned char* const rt = s_dyn + row * PT + c * (int)sizeof(T);
+        T U[NV];
 #pragma unroll
-        for (int m = 0; m < NV; m++) xd[m] = __ldcg(src + m * TC);
-      };
-      // old-state half of step t's term: comput_DFn's F(U)n (sub_LU_SGS.f90:135-157), in the flux
-      // precision; the neighbour's U, Lc, Lv are in the previous step's record, the face's normal
-      // and area in this step's
-      using DFT = T;
-      DFT Ub[NV], F1[NV], n1 = 0, n2 = 0, n3 = 0;
-      double Sd = 0.0, wLc = 0.0, Lvd = 0.0;
-      bool hd = false;
-      auto prep = [&](int t) {
-        hd = on_at(t) && has(d, cell_i(t));
-        if (!hd) return;
-        const unsigned char* so = stage(seq0 + t + 1);
-        const unsigned char* sn = stage(seq0 + t);
-        const T* Nn = (const T*)(so + S.dyn_bytes + S.o_n);
-        const T* Sa = (const T*)(so + S.dyn_bytes + (UPPER ? S.o_Sup : S.o_Slo));
-        n1 = (DFT)Nn[(3 * d) * TC + c];
-        n2 = (DFT)Nn[(3 * d + 1) * TC + c];
-        n3 = (DFT)Nn[(3 * d + 2) * TC + c];
-        Sd = (double)Sa[d * TC + c];
-        wLc = w * (double)((const T*)(sn + S.o_Lc))[d * E + en];
-        Lvd = (double)((const T*)(sn + S.o_Lv))[d * E + en];
-        const double* Un = (const double*)(sn + S.o_U);
+        for (int m = 0; m < NV; m++) {
+          const double u = *reinterpret_cast<const double*>(r8 + SM::U + m * ROWS * PB);
+          U[m] = (T)(m >= 5 ? clamp0(u) : u);
+        }
+        const double vol = *reinterpret_cast<const double*>(r8 + SM::VOL);
+        const double dtd = (double)*reinterpret_cast<const T*>(rt + SM::DT);
+        double lc[3], lvd[3];
 #pragma unroll
-        for (int m = 0; m < NV; m++) Ub[m] = (DFT)Un[m * E + en];
-        const DFT g1 = (DFT)(gamma - 1.0), half = (DFT)0.5;
-        const DFT un1 = (Ub[1] * n1 + Ub[2] * n2 + Ub[3] * n3) / Ub[0];
-        const DFT p1 = g1 * (Ub[4] - half * (sq(Ub[1]) + sq(Ub[2]) + sq(Ub[3])) / Ub[0]);
-        F1[0] = Ub[0] * un1;
-        F1[1] = Ub[1] * un1 + p1 * n1;
-        F1[2] = Ub[2] * un1 + p1 * n2;
-        F1[3] = Ub[3] * un1 + p1 * n3;
-        F1[4] = (Ub[4] + p1) * un1;
+        for (int m = 0; m < 3; m++) {
+          lc[m] = (double)*reinterpret_cast<const T*>(rt + SM::LC + m * ROWS * PT);
+          lvd[m] = (double)*reinterpret_cast<const T*>(rt + SM::LV + m * ROWS * PT);
+        }
+        const T r0 = rcp_rn(U[0]);
+        const T kin = half * sq3(U);
+        T ke = div_by(kin, U[0], r0);
+        // the diagonal (sub_LU_SGS.f90:50-62, 90-92)
+        double vdt = div_by(vol, dtd, rcp_rn(dtd));
+        if (bad_den(U[0]) || bad_num(expo(kin), kin) || bad_den(dtd) || bad_num(expo(vol), 0.0)) { ke = kin / U[0]; vdt = vol / dtd; }
+        const T ei = U[4] - ke;
+        const double a0 = vdt + w * (lc[0] + lc[1] + lc[2]);
+        double al = a0, als = a0;
+        if (visc) {
+          const double lv = lvd[0] + lvd[1] + lvd[2];
+          al = al + 2.0 * lv;
+          als = als + 2.0 * lv;
+          if (NV == 6) {  // lower: + (Lv sum); upper: + Lv1 + Lv2 + Lv3 term by term
+            if (!UPPER) als = als + lv;
+            else als = als + lvd[0] + lvd[1] + lvd[2];
+          }
+        }
+        if (dual) {  // dual time: + Sfac1 vol (sub_LU_SGS.f90:39, 92)
+          al = al + sfac1 * vol;
+          als = als + sfac1 * vol;
+        }
+        double ra = rcp_rn(al), ras = NV == 6 ? rcp_rn(als) : 0.0;
+        if (bad_den(al) || (NV == 6 && bad_den(als))) { ra = 1.0 / al; ras = 1.0 / als; }
+        mb_wait(empty0 + 8 * (n % SLOTS), (n / SLOTS + 1) & 1, L.err);  // the slot's last readers are done
+        double* const pa = reinterpret_cast<double*>(sl + SM::AL) + c;
+        if (FP64) {
+          pa[0] = al; pa[TC] = ra;
+          if (NV == 6) { pa[AS5 * TC] = als; pa[(AS5 + 1) * TC] = ras; }
+        } else {
+          pa[0] = ra;
+          if (NV == 6) pa[(NA - 1) * TC] = ras;
 #pragma unroll
-        for (int m = 5; m < NV; m++) F1[m] = Ub[m] * un1;
-      };
-      bool ok = wait_rec(seq0);
-      ok &= wait_rec(seq0 + 1);
-      if (!ok) atomicExch(L.err, 1);
-      prep(0);
-      double xdu[NV];
+          for (int m = 0; m < NV; m++) reinterpret_cast<T*>(sl + SM::SU)[m * TC + c] = U[m];
+        }
+        reinterpret_cast<T*>(sl + SM::Q)[c] = r0;
+        reinterpret_cast<T*>(sl + SM::Q)[TC + c] = ei;
+        __syncwarp();
+        if (lane == 0) mb_arrive(fullP + 8 * (n % SLOTS));
+      }
+    } else if (role < 7) {
+      // ------------------------------------------------------------------ input rows in, DU out
+      constexpr int LW = 2 * RW, CR = 32 / WB, NR = TC / CR / LW;  // loader warps; columns per request; requests per stream and warp
+      const int lw = (tid - 5 * TC) / 32, iw = lane % WB;
+      long long cb[NR], bb[NR], fb[NR];
+      int sk[NR], col[NR];
+      bool act[NR], dj[NR], dk[NR];
 #pragma unroll
-      for (int m = 0; m < NV; m++) xdu[m] = 0.0;
-      __syncthreads();   // B0: the helper's first waits are done
-      if (xt && hd) load_x(0, xdu);
-      for (int t = 0; t < nsteps; t++) {
-        __syncthreads();   // B1: step t-1's DU is in s_du
-        double nxdu[NV];
+      for (int r = 0; r < NR; r++) {
+        col[r] = (lw * NR + r) * CR + lane / WB;
+        const int qj = col[r] % TJ, qk = col[r] / TJ;
+        const int jj = UPPER ? (tl.j0 + TJ - 1 - qj) : (tl.j0 + qj), kk = UPPER ? (tl.k0 + TK - 1 - qk) : (tl.k0 + qk);
+        act[r] = jj >= 1 && jj <= nym && kk >= 1 && kk <= nzm;
+        // idle columns and steps load a cell of the block that nobody uses
+        const int jc = min(max(jj, 1), nym), kc = min(max(kk, 1), nzm);
+        sk[r] = qj + qk;
+        dj[r] = jc > 1;
+        dk[r] = kc > 1;
+        cb[r] = B.ocell - 1 + (long long)nxm * ((jc - 1) + (long long)nym * (kc - 1));
+        bb[r] = B.obox + 3 + (long long)B.NX * ((jc + 3) + (long long)B.NY * (kc + 3));
+        fb[r] = B.oface - 1 + (long long)B.nx * ((jc - 1) + (long long)B.ny * (kc - 1));
+      }
+      const unsigned base = (unsigned)__cvta_generic_to_shared(s_dyn);
+      const long long sj = B.nx, sk2 = (long long)B.nx * B.ny;
+      for (int wb = 0; wb < nblk + 2; wb++) {
+        const unsigned gb = ib + wb;
+        const int row = (int)(gb & 1) * WB + iw;
+        if (wb >= 2) {  // block wb - 2 is done: its DU to memory, then its rows are free
+          mb_wait(emptyR + 8 * (gb & 1), ((gb - 2) >> 1) & 1, L.err);
+          const int t = (wb - 2) * WB + iw;
 #pragma unroll
-        for (int m = 0; m < NV; m++) nxdu[m] = 0.0;
-        if (xt && on_at(t + 1) && has(d, cell_i(t + 1))) load_x(t + 1, nxdu);   // ready since the wait before B1
-        if (hd) {
-          double DUn[NV];
+          for (int r = 0; r < NR; r++) {
+            const int il = t - sk[r];
+            if (act[r] && il >= 0 && il < nxm) {
+              double* const o = A.DU + cb[r] + (UPPER ? nxm - il : il + 1);
+              const double* const v = reinterpret_cast<const double*>(s_dyn + SM::R + row * PB) + col[r];
 #pragma unroll
-          for (int m = 0; m < NV; m++) DUn[m] = xt ? xdu[m] : s_du[(t + 1) & 1][m][cn];
-          DFT U2[NV];
+              for (int m = 0; m < NV; m++) o[m * tc] = v[m * ROWS * (PB / 8)];
+            }
+          }
+        }
+        if (wb >= nblk) continue;
+        cta_bar_id<2, 2 * TC>();  // every loader warp has read the rows
+        const int t = wb * WB + iw;
 #pragma unroll
-          for (int m = 0; m < NV; m++) U2[m] = (DFT)((double)Ub[m] + DUn[m]);
-          const DFT g1 = (DFT)(gamma - 1.0), half = (DFT)0.5;
-          const DFT un2 = (U2[1] * n1 + U2[2] * n2 + U2[3] * n3) / U2[0];
-          const DFT pp2 = g1 * (U2[4] - half * (sq(U2[1]) + sq(U2[2]) + sq(U2[3])) / U2[0]);
-          DFT DF[NV];
-          DF[0] = U2[0] * un2 - F1[0];
-          DF[1] = (U2[1] * un2 + pp2 * n1) - F1[1];
-          DF[2] = (U2[2] * un2 + pp2 * n2) - F1[2];
-          DF[3] = (U2[3] * un2 + pp2 * n3) - F1[3];
-          DF[4] = (U2[4] + pp2) * un2 - F1[4];
-#pragma unroll
-          for (int m = 5; m < NV; m++) DF[m] = U2[m] * un2 - F1[m];
+        for (int r = 0; r < NR; r++) {
+          if (wb >= 2) __nanosleep(LU5_PACE);  // leaves the load path to D's reads in between
+          const int il = min(max(t - sk[r], 0), nxm - 1), i = UPPER ? nxm - il : il + 1;
+          const unsigned d8 = base + row * PB + col[r] * 8, dt_ = base + row * PT + col[r] * (int)sizeof(T);
+          const double* const pU = A.U + bb[r] + i;
+          const long long ci = cb[r] + i, f = fb[r] + i;
 #pragma unroll
           for (int m = 0; m < NV; m++) {
-            double v;
-            if (MIXED) {   // the off-diagonal products in FP32 (the accumulation stays FP64)
-              const float du = (float)DUn[m];
-              float x;
-              if (!UPPER) x = 0.5f * ((float)DF[m] * (float)Sd + (float)wLc * du);
-              else x = -(0.5f * ((float)DF[m] * (float)Sd - (float)wLc * du));
-              if (visc) x = x + (float)Lvd * du;
-              v = (double)x;
-            } else {
-              if (!UPPER) v = 0.5 * ((double)DF[m] * Sd + wLc * DUn[m]);
-              else v = -(0.5 * ((double)DF[m] * Sd - wLc * DUn[m]));
-              if (visc) v = v + Lvd * DUn[m];
-            }
-            s_acc[d][m][c] = v;
+            cp_elem(d8 + SM::U + m * ROWS * PB, pU + m * tb);
+            if (UPPER) cp_elem(d8 + SM::R + m * ROWS * PB, A.DU + ci + m * tc);  // DU* of the lower sweep
+            else cp_elem(base + SM::R + (m * ROWS + row) * PB + col[r] * (int)sizeof(T), A.Res + ci + m * tc);
           }
-        } else if (on_at(t)) {
+          cp_elem(d8 + SM::VOL, A.vold + ci);
+          cp_elem(dt_ + SM::DT, A.dt + ci);
+          // the downstream face of direction m: its normal is the lower face's of the downstream cell,
+          // its area the lower face's (lower sweep) or the upper face's of that cell (upper sweep,
+          // sub_LU_SGS.f90:96-97); without a downstream cell the term is not used
 #pragma unroll
-          for (int m = 0; m < NV; m++) s_acc[d][m][c] = 0.0;
+          for (int m = 0; m < 3; m++) {
+            cp_elem(dt_ + SM::LC + m * ROWS * PT, A.Lc + ci + m * tc);
+            cp_elem(dt_ + SM::LV + m * ROWS * PT, A.Lv + ci + m * tc);
+            const long long st = m == 0 ? 1 : (m == 1 ? sj : sk2);
+            const long long fn = UPPER ? ((m == 0 ? i > 1 : (m == 1 ? dj[r] : dk[r])) ? f - st : f) : f + st;
+            const T* const pn = A.M + (M_NI1 + 3 * m) * tf + fn;
+            cp_elem(dt_ + SM::N + (3 * m) * ROWS * PT, pn);
+            cp_elem(dt_ + SM::N + (3 * m + 1) * ROWS * PT, pn + tf);
+            cp_elem(dt_ + SM::N + (3 * m + 2) * ROWS * PT, pn + 2 * tf);
+            cp_elem(dt_ + SM::S + m * ROWS * PT, A.M + (M_SI + m) * tf + (UPPER ? f : f + st));
+          }
         }
-        lu5_bar_compute<4 * TC>();   // B2: the terms and the diagonal of step t are in shared memory
-        if (on_at(t)) store(d, t, finish(d, t));
-        if (t + 1 < nsteps) {
-          if (on_at(t + 1) && !wait_rec(seq0 + t + 2)) atomicExch(L.err, 1);
-          prep(t + 1);
-        }
+        cp_arrive(fullR + 8 * (gb & 1));
+      }
+    } else {
+      // ------------------------------------------------------------------ terms from the upstream tiles
+      constexpr int EPL = (NV * (TC / 2 + 2) + 31) / 32, W = EPL > 4 ? 2 : 4;  // words per lane and step; steps polled at once
+      const bool up_j = UPPER ? J < nJ - 1 : J > 0, up_k = UPPER ? K < nK - 1 : K > 0;
+      long long* src[EPL];
+      int lo[EPL], stride[EPL], dst[EPL];
+      const int step_j = first + (UPPER ? J + 1 : J - 1) + nJ * K, step_k = first + J + nJ * (UPPER ? K + 1 : K - 1);
 #pragma unroll
-        for (int m = 0; m < NV; m++) xdu[m] = nxdu[m];
+      for (int e = 0; e < EPL; e++) {
+        const int x = lane + 32 * e;
+        src[e] = nullptr; lo[e] = 0; stride[e] = 0; dst[e] = 0;
+        if (x < NV * TK) {  // j edge: the upstream tile's column (TJ - 1, ek), TJ - 1 steps later there
+          const int m = x / TK, ek = x % TK, kk = UPPER ? tl.k0 + TK - 1 - ek : tl.k0 + ek;
+          if (up_j && kk >= 1 && kk <= nzm) {
+            src[e] = L.edge + L.edge_off[step_j] + ((long long)(TJ - 1) * NV + m) * TK + ek;
+            stride[e] = NV * TK; lo[e] = ek; dst[e] = (1 * NV + m) * SM::AS + TC + ek * TJ + TJ - 1;
+          }
+        } else if (x < NV * (TJ + TK)) {  // k edge
+          const int m = (x - NV * TK) / TJ, ej = (x - NV * TK) % TJ, jj = UPPER ? tl.j0 + TJ - 1 - ej : tl.j0 + ej;
+          if (up_k && jj >= 1 && jj <= nym) {
+            src[e] = L.edge + L.edge_off[step_k] + (long long)nsteps * NV * TK + ((long long)(TK - 1) * NV + m) * TJ + ej;
+            stride[e] = NV * TJ; lo[e] = ej; dst[e] = (2 * NV + m) * SM::AS + TC + TC - TJ + ej;
+          }
+        }
+      }
+      long long spins = 0;
+      bool gave_up = false;
+      int t = 0;
+      while (t < nsteps) {
+        long long v[W][EPL];
+        int ready = 0;
+        bool all = true;
+#pragma unroll
+        for (int g = 0; g < W; g++)
+#pragma unroll
+          for (int e = 0; e < EPL; e++) {
+            const int il = t + g - lo[e];
+            v[g][e] = 0;
+            if (src[e] && il >= 0 && il < nxm && !gave_up) v[g][e] = ld_word(src[e] + (long long)(t + g) * stride[e]);
+          }
+#pragma unroll
+        for (int g = 0; g < W; g++) {
+          bool here = t + g < nsteps;
+#pragma unroll
+          for (int e = 0; e < EPL; e++) here &= v[g][e] != LU5_EMPTY;
+          all = all && __all_sync(0xffffffffu, here);
+          ready += all ? 1 : 0;
+        }
+        if (ready == 0) {
+          if (++spins > L.spin_limit) {
+            gave_up = true;
+            if (lane == 0) atomicExch(L.err, 1);
+          }
+          continue;
+        }
+        spins = 0;
+#pragma unroll
+        for (int g = 0; g < W; g++) {
+          if (g >= ready) break;
+          const unsigned n = it + t + g;
+          double* const acc = reinterpret_cast<double*>(slot_of(n) + SM::ACC);
+          mb_wait(empty0 + 8 * (n % SLOTS), (n / SLOTS + 1) & 1, L.err);
+#pragma unroll
+          for (int e = 0; e < EPL; e++) {
+            const int il = t + g - lo[e];
+            if (src[e] && il >= 0 && il < nxm) {
+              acc[dst[e]] = __longlong_as_double(v[g][e]);
+              st_word(src[e] + (long long)(t + g) * stride[e], LU5_EMPTY);
+            }
+          }
+          __syncwarp();
+          if (lane == 0) mb_arrive(fullE + 8 * (n % SLOTS));
+        }
+        t += ready;
       }
     }
-    __syncthreads();   // the tile's last step is done everywhere
-    if (tid == HT) st_release(L.progress + my, nsteps);
-    seq0 += nrecs;
+    it += nsteps;
+    ib += nblk;
   }
 }
 
-template <class T, int NV, bool UPPER, int TC>
-inline void lu_wave5_prepare(const LuStream& S) {
-  cudaFuncSetAttribute(k_lusgs_wave5<T, NV, UPPER, TC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lu5_smem<T, NV, TC>(S, UPPER));
+template <class T, int NV, int TC>
+inline void lu_wave5_prepare() {
+  cudaFuncSetAttribute(k_lusgs_wave5<T, NV, false, TC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lu5_smem<T, NV, false, TC>());
+  cudaFuncSetAttribute(k_lusgs_wave5<T, NV, true, TC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lu5_smem<T, NV, true, TC>());
 }
 
 }  // namespace ocfd

@@ -83,11 +83,8 @@ class RunnerT : public Runner {
       ns_prepare<true, -1, -1>();
       ns_prepare<false, -1, -1>();
     }
-    if (I.lus) {
-      S_ = *I.lus;
-      if (L_.TJ * L_.TK == 64) { lu_wave5_prepare<T, NV, false, 64>(S_); lu_wave5_prepare<T, NV, true, 64>(S_); }
-      else { lu_wave5_prepare<T, NV, false, 32>(S_); lu_wave5_prepare<T, NV, true, 32>(S_); }
-    }
+    lu_wave5_prepare<T, NV, 32>();
+    lu_wave5_prepare<T, NV, 64>();
   }
 
   void residual(cudaStream_t st, bool lusgs) override {
@@ -245,17 +242,14 @@ class RunnerT : public Runner {
     } else {
       if (upper && I_.lu_version == 4 && I_.lu_fused) return;  // ran with the lower sweep's launch
       if (!upper) cudaMemsetAsync(L_.counter, 0, 2 * sizeof(int), st);
-      cudaMemsetAsync(L_.progress, 0, sizeof(int) * L_.ntiles, st);
+      if (I_.lu_version != 5) cudaMemsetAsync(L_.progress, 0, sizeof(int) * L_.ntiles, st);
       if (I_.lu_version == 5) {
-        const int TC = L_.TJ * L_.TK;
-        const int g = I_.lu5_grid[upper ? 1 : 0];
-        if (!upper) k_lu_pack_dyn<T, NV><<<dim3(8, L_.ntiles), 256, 0, st>>>(A, S_, L_.TJ, L_.TK);
-        if (TC == 64) {
-          if (!upper) k_lusgs_wave5<T, NV, false, 64><<<g, 4 * 64 + 32, lu5_smem<T, NV, 64>(S_, false), st>>>(A, L_, S_);
-          else k_lusgs_wave5<T, NV, true, 64><<<g, 4 * 64 + 32, lu5_smem<T, NV, 64>(S_, true), st>>>(A, L_, S_);
+        if (I_.lu_tc == 64) {
+          if (!upper) k_lusgs_wave5<T, NV, false, 64><<<I_.lu_grid, lu5_threads<64>(), lu5_smem<T, NV, false, 64>(), st>>>(A, L_);
+          else k_lusgs_wave5<T, NV, true, 64><<<I_.lu_grid, lu5_threads<64>(), lu5_smem<T, NV, true, 64>(), st>>>(A, L_);
         } else {
-          if (!upper) k_lusgs_wave5<T, NV, false, 32><<<g, 4 * 32 + 32, lu5_smem<T, NV, 32>(S_, false), st>>>(A, L_, S_);
-          else k_lusgs_wave5<T, NV, true, 32><<<g, 4 * 32 + 32, lu5_smem<T, NV, 32>(S_, true), st>>>(A, L_, S_);
+          if (!upper) k_lusgs_wave5<T, NV, false, 32><<<I_.lu_grid, lu5_threads<32>(), lu5_smem<T, NV, false, 32>(), st>>>(A, L_);
+          else k_lusgs_wave5<T, NV, true, 32><<<I_.lu_grid, lu5_threads<32>(), lu5_smem<T, NV, true, 32>(), st>>>(A, L_);
         }
       } else if (I_.lu_version == 2) {
         if (!upper) k_lusgs_wave<T, NV, false><<<I_.lu_grid, 64, 0, st>>>(A, L_);
@@ -390,7 +384,7 @@ class RunnerT : public Runner {
       if (I_.turb == 2 && NV == 6) res += I_.sa_fused ? 3 : 6;  // sa_pre, (tile | 3 fluxes + res), mu_finish
       else if (I_.turb == 3 && NV == 7) res += 11;
     }
-    int lu = I_.lu_planes ? 2 * (I_.max_plane - 2) : (I_.lu_version == 5 ? 3 : (I_.lu_version == 4 && I_.lu_fused ? 1 : 2));
+    int lu = I_.lu_planes ? 2 * (I_.max_plane - 2) : (I_.lu_version == 4 && I_.lu_fused ? 1 : 2);
     int upd = 1 + 1 + (NV == 6 ? 3 : 0);
     int nbc = 0;
     for (int r = 0; r < I_.nround; r++) nbc += I_.bc_rounds[3 * r + 2] > 0;
@@ -402,10 +396,6 @@ class RunnerT : public Runner {
     else n = 1 + 3 * (res + upd + bch);
     if (NV >= 6) n += 1;
     return n;
-  }
-
-  void lu5_pack_geo(cudaStream_t st) override {
-    if (I_.lus) k_lu_pack_geo<T><<<dim3(8, L_.ntiles), 256, 0, st>>>(A_, S_, L_.TJ, L_.TK);
   }
 
   void dual_init(cudaStream_t st) override { k_dual_init<T, NV><<<grid_of((long long)NV * A_.tot_box), 256, 0, st>>>(A_); }
@@ -439,7 +429,6 @@ class RunnerT : public Runner {
   Arena<T> A_;
   RunInfo I_;
   LuArgs L_{};
-  LuStream S_{};
   int ns_grid_[5] = {1, 1, 1, 1, 1};  // CTAs of k_ns_tile per instantiation (resident CTAs, at most the tiles)
   int sa_grid_ = 1;                 // CTAs of k_sa_tile
   cudaStream_t st2_ = nullptr;      // the second stream of a forked residual (RunInfo::res_streams)

@@ -8,7 +8,6 @@
 namespace ocfd {
 
 struct LuArgs;
-struct LuStream;
 
 struct RunInfo {
   int nvar, time_method, viscous, turb;
@@ -19,9 +18,7 @@ struct RunInfo {
   const LuArgs* lu;       // wavefront tables (host copy of the kernel argument)
   int lu_grid;            // CTAs of the wavefront kernel
   int lu_version;         // 2: one thread per column; 3: four thread groups per column, staged by element; 4: staged by sector;
-                          // 5: inputs packed in sweep order, one bulk copy per step (lus)
-  const LuStream* lus;    // version 5: record layout and buffers (host copy of the kernel argument)
-  int lu5_grid[2];        // version 5: CTAs of the lower / upper sweep (resident CTAs, at most the tiles)
+                          // 5: terms evaluated by the producing cell, one warp role per task (lusgs5.cuh)
   int lu_tc;              // columns per tile (32 or 64)
   int lu_fused;           // version 4: both sweeps in one launch (k_lusgs_wave4_ul)
   int recon_prim;         // 1: every solve reconstructs primitive variables
@@ -83,8 +80,6 @@ class Runner {
   virtual void norms(cudaStream_t st, double* part, double* out, unsigned long long* nan_at) = 0;
   // force partial sums: 9 doubles per wall chunk
   virtual void forces(cudaStream_t st, double* part) = 0;
-  // version-5 LU-SGS: the static geometry records (once, after the geometry is computed)
-  virtual void lu5_pack_geo(cudaStream_t st) = 0;
   // AoS Fortran U(NV, box) of one block <-> device planes
   virtual void scatter_state(cudaStream_t st, int blk, const double* aos, long long box_b) = 0;
   virtual void gather_state(cudaStream_t st, int blk, double* aos, long long box_b) = 0;

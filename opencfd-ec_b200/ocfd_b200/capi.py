@@ -228,11 +228,11 @@ class Solver:
         return int(lib().ocfd_launches_per_step(self.h))
 
     def lu_tile_width(self):
-        """Columns per CTA tile of the LU-SGS sweeps, as picked by the creation-time autotuner."""
+        """Columns per CTA tile of the LU-SGS sweeps."""
         return int(lib().ocfd_lu_tile_width(self.h))
 
     def lu_kernel_version(self):
-        """LU-SGS wavefront kernel version in use (3 or 4; 2 with OCFD_LU_V2), as picked at creation."""
+        """LU-SGS wavefront kernel version in use (5 unless a switch selects another)."""
         return int(lib().ocfd_lu_kernel_version(self.h))
 
     def lu_one_launch(self):
