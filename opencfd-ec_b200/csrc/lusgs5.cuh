@@ -61,32 +61,13 @@ constexpr int LU5_PACE = 300;  // ns between a loader warp's requests: keeps bur
 constexpr long long LU5_EMPTY = -1LL;  // the sentinel of an edge word
 
 // ---- division by a shared reciprocal -------------------------------------------------------
-// RN(1/b) for |b| in 2^-511 .. 2^511: a 20-bit seed, one cubic step (relative error below 2^-58), one
-// correction; for a mantissa of all ones, the one the correction can miss, the result is known
-// (freestream densities one unit below 1 meet it)
-__device__ __forceinline__ double rcp_rn(double b) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
-  double e = __fma_rn(-b, y, 1.0);
-  e = __fma_rn(e, e, e);
-  y = __fma_rn(y, e, y);
-  e = __fma_rn(-b, y, 1.0);
-  y = __fma_rn(y, e, y);
-  const bool ones = __double2loint(b) == -1 && (__double2hiint(b) & 0xfffff) == 0xfffff;
-  return ones ? __hiloint2double(__double2hiint(y) & 0xfff00000, 1) : y;
-}
+// (rcp_rn, div_by and expo of double are in physics.cuh)
 __device__ __forceinline__ float rcp_rn(float b) { return __frcp_rn(b); }
-// RN(x / b) from r = RN(1/b)
-__device__ __forceinline__ double div_by(double x, double b, double r) {
-  const double q = __dmul_rn(x, r);
-  return __fma_rn(__fma_rn(-b, q, x), r, q);
-}
 __device__ __forceinline__ float div_by(float x, float b, float r) {
   const float q = __fmul_rn(x, r);
   return __fmaf_rn(__fmaf_rn(-b, q, x), r, q);
 }
 // the exponent word of |x|, and whether operands lie outside the range div_by is exact in
-__device__ __forceinline__ unsigned expo(double x) { return (unsigned)__double2hiint(x) & 0x7fffffffu; }
 __device__ __forceinline__ unsigned expo(float x) { return (unsigned)__float_as_int(x) & 0x7fffffffu; }
 __device__ __forceinline__ bool bad_den(double b) { return expo(b) - 0x20000000u > 0x3fc00000u; }  // |b| in 2^-511 .. 2^509
 __device__ __forceinline__ bool bad_num(unsigned e, double) { return e > 0x5fc00000u; }

@@ -636,9 +636,11 @@ struct InvFluxOcc { static constexpr int value = sizeof(T) == 8 ? 3 : INV_FLUX_M
 // straight-line path (the five reconstructions without a switch between them, free to interleave)
 // and the flux switch folds; boundary faces keep the general path.
 // CTAs per SM: FP64 3 (80 registers); the FP64 MUSCL3 specialisation 2 (about 120 registers, no
-// spills: config 1 residual phase 0.099 -> 0.094 ms; WENO5 is faster at 3, 1.85 against 2.00 ms)
+// spills: config 1 residual phase 0.099 -> 0.094 ms; WENO5 is faster at 3, 1.55 against 1.60 ms)
 template <class T, int ISCH>
 struct InvFluxOccS { static constexpr int value = (sizeof(T) == 8 && ISCH == S_MUSCL3) ? 2 : InvFluxOcc<T>::value; };
+template <class T, int DIR, bool PRIM, int IFLUX>
+__device__ __noinline__ void inv_face_plain(const Arena<T>& A, int b, int i, int j, int k, long long g, T* Fo);
 // one face of direction DIR: its five inviscid flux components (the face's Fi plane entries)
 template <class T, int DIR, bool PRIM, int ISCH, int IFLUX>
 __device__ __forceinline__ void inv_face(const Arena<T>& A, const BlkD& B, const SolveP& s, int b, int i, int j, int k, long long g,
@@ -658,6 +660,11 @@ __device__ __forceinline__ void inv_face(const Arena<T>& A, const BlkD& B, const
   long long c0 = bix(B, i - 4 * di, j - 4 * dj, k - 4 * dk);
   const long long st = DIR == 0 ? 1 : (DIR == 1 ? (long long)B.NX : (long long)B.NX * B.NY);
   T UL[5], UR[5];
+  // the FP64 WENO5 / MUSCL3 + Roe instantiations divide through reciprocals, without branches (the
+  // same bits): 57 divisions a WENO5 face, each a subroutine that kept the five variables from
+  // overlapping (config 2 residual phase 1.74 -> 1.55 ms, step 2.87 -> 2.71 ms).  A face with operands
+  // outside that division's range is evaluated again out of line
+  constexpr bool FAST = sizeof(T) == 8 && (ISCH == S_WENO5 || ISCH == S_MUSCL3) && IFLUX == F_ROE;
   if ((PRIM || s.recon == 0) && ISCH >= 0 && scheme == ISCH) {
 #pragma unroll
     for (int m = 0; m < 5; m++) {
@@ -665,7 +672,14 @@ __device__ __forceinline__ void inv_face(const Arena<T>& A, const BlkD& B, const
       T u[8];
 #pragma unroll
       for (int q = 0; q < 8; q++) u[q] = A.P[pl * tb + c0 + q * st];
-      scheme_LR(u, ISCH < 0 ? 0 : ISCH, UL[m], UR[m]);
+      if constexpr (FAST && ISCH == S_WENO5) {
+        UL[m] = weno5_fast(u[1], u[2], u[3], u[4], u[5]);
+        UR[m] = weno5_fast(u[6], u[5], u[4], u[3], u[2]);
+      } else if constexpr (FAST) {
+        muscl3_fast(u, UL[m], UR[m]);
+      } else {
+        scheme_LR(u, ISCH < 0 ? 0 : ISCH, UL[m], UR[m]);
+      }
     }
   } else if (PRIM || s.recon == 0) {
     T u[8];
@@ -725,7 +739,7 @@ __device__ __forceinline__ void inv_face(const Arena<T>& A, const BlkD& B, const
       UR[4] = (QR[4] - (UR[1] * QR[1] + UR[2] * QR[2] + UR[3] * QR[3]) * T(0.5)) * (gm - T(1));
     }
   }
-  if (s.positivity == 1) {  // first-order fallback (sub_Residual.f90:283-299)
+  auto positivity = [&]() {  // first-order fallback (sub_Residual.f90:283-299)
     const T lz = T(1.e-20);
     if (UL[0] <= lz || UL[4] <= lz) {
       long long cl = c0 + 3 * st;
@@ -735,16 +749,32 @@ __device__ __forceinline__ void inv_face(const Arena<T>& A, const BlkD& B, const
       long long cr = c0 + 4 * st;
       UR[0] = A.P[P_D * tb + cr]; UR[1] = A.P[P_U * tb + cr]; UR[2] = A.P[P_V * tb + cr]; UR[3] = A.P[P_W * tb + cr]; UR[4] = A.P[P_P * tb + cr];
     }
-  }
+  };
+  if (s.positivity == 1) positivity();
   T s1x = A.M[(M_NI1 + 3 * DIR) * tf + g], s1y = A.M[(M_NI2 + 3 * DIR) * tf + g], s1z = A.M[(M_NI3 + 3 * DIR) * tf + g];
   T s2x = A.M[(M_TI + 3 * DIR) * tf + g], s2y = A.M[(M_TI + 3 * DIR + 1) * tf + g], s2z = A.M[(M_TI + 3 * DIR + 2) * tf + g];
   T s3x = s1y * s2z - s1z * s2y, s3y = s1z * s2x - s1x * s2z, s3z = s1x * s2y - s1y * s2x;
   T QL[5], QR[5], F0[5];
-  QL[0] = UL[0]; QL[1] = UL[1] * s1x + UL[2] * s1y + UL[3] * s1z; QL[2] = UL[1] * s2x + UL[2] * s2y + UL[3] * s2z;
-  QL[3] = UL[1] * s3x + UL[2] * s3y + UL[3] * s3z; QL[4] = UL[4];
-  QR[0] = UR[0]; QR[1] = UR[1] * s1x + UR[2] * s1y + UR[3] * s1z; QR[2] = UR[1] * s2x + UR[2] * s2y + UR[3] * s2z;
-  QR[3] = UR[1] * s3x + UR[2] * s3y + UR[3] * s3z; QR[4] = UR[4];
-  flux_1d(QL, QR, F0, T(s.gamma), IFLUX >= 0 ? IFLUX : s.flux);
+  auto rotate = [&]() {
+    QL[0] = UL[0]; QL[1] = UL[1] * s1x + UL[2] * s1y + UL[3] * s1z; QL[2] = UL[1] * s2x + UL[2] * s2y + UL[3] * s2z;
+    QL[3] = UL[1] * s3x + UL[2] * s3y + UL[3] * s3z; QL[4] = UL[4];
+    QR[0] = UR[0]; QR[1] = UR[1] * s1x + UR[2] * s1y + UR[3] * s1z; QR[2] = UR[1] * s2x + UR[2] * s2y + UR[3] * s2z;
+    QR[3] = UR[1] * s3x + UR[2] * s3y + UR[3] * s3z; QR[4] = UR[4];
+  };
+  rotate();
+  if constexpr (FAST) {
+    ExRange x;
+    flux_roe_fast(QL, QR, F0, s.gamma, x);
+    if (x.bad()) {
+      T Fp[5];
+      inv_face_plain<T, DIR, PRIM, IFLUX>(A, b, i, j, k, g, Fp);
+#pragma unroll
+      for (int m = 0; m < 5; m++) Fo[m] = Fp[m];
+      return;
+    }
+  } else {
+    flux_1d(QL, QR, F0, T(s.gamma), IFLUX >= 0 ? IFLUX : s.flux);
+  }
   T S = A.M[(M_SI + DIR) * tf + g];
   Fo[0] = -F0[0] * S;
   Fo[1] = -(F0[1] * s1x + F0[2] * s2x + F0[3] * s3x) * S;
@@ -753,8 +783,15 @@ __device__ __forceinline__ void inv_face(const Arena<T>& A, const BlkD& B, const
   Fo[4] = -F0[4] * S;
 }
 
+// the same face by plain division (out of line: it is hardly ever taken)
+template <class T, int DIR, bool PRIM, int IFLUX>
+__device__ __noinline__ void inv_face_plain(const Arena<T>& A, int b, int i, int j, int k, long long g, T* Fo) {
+  const BlkD& B = A.blk[b];
+  inv_face<T, DIR, PRIM, -1, IFLUX>(A, B, A.sp[B.solve], b, i, j, k, g, Fo);
+}
+
 template <class T, int DIR, bool PRIM = false, int ISCH = -1, int IFLUX = -1>
-__global__ void __launch_bounds__(256, InvFluxOccS<T, ISCH>::value) k_inv_flux(Arena<T> A) {
+__global__ void __launch_bounds__(256, InvFluxOccS<T, ISCH>::value) k_inv_flux(const __grid_constant__ Arena<T> A) {
   const long long tf = A.tot_face;
   OCFD_GRID_STRIDE(g, tf) {
     int b = find_blk_h(A.pre_face, A.hint_face, A.nblk, g);
@@ -1133,7 +1170,7 @@ __device__ __forceinline__ void tile_visc_zero(const Arena<T>& A, const BlkD& B,
 template <class T, int ISCH, bool INV>
 struct NsTileOcc { static constexpr int value = INV ? InvFluxOccS<T, ISCH>::value : OCFD_MEM_MINB; };
 template <class T, bool PRIM, int ISCH, int IFLUX, bool VISC, bool INV = true>
-__global__ void __launch_bounds__(256, NsTileOcc<T, ISCH, INV>::value) k_ns_tile(Arena<T> A) {
+__global__ void __launch_bounds__(256, NsTileOcc<T, ISCH, INV>::value) k_ns_tile(const __grid_constant__ Arena<T> A) {
   extern __shared__ __align__(16) unsigned char ns_smem[];
   T* Fs = reinterpret_cast<T*>(ns_smem);
   T* Rs = Fs + 5 * A.tile_maxf;
