@@ -183,7 +183,10 @@ __global__ void __launch_bounds__(7 * TC + 32, 1) k_lusgs_wave5(Arena<T> A, LuAr
     if (tid == 0) s_tile = atomicAdd(&L.counter[UPPER ? 1 : 0], 1);
     __syncthreads();
     const int q = s_tile;
-    if (q >= L.ntiles) break;
+    if (q >= L.ntiles) {  // the last CTA to ask leaves the counter at 0 for the next sweep
+      if (tid == 0 && q == L.ntiles + (int)gridDim.x - 1) L.counter[UPPER ? 1 : 0] = 0;
+      break;
+    }
     const LuTile tl = UPPER ? L.rtiles[q] : L.tiles[q];
     const BlkD& B = A.blk[tl.blk];
     const SolveP& s = A.sp[B.solve];

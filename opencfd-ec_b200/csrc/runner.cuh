@@ -241,8 +241,10 @@ class RunnerT : public Runner {
       else for (int p = I_.max_plane; p >= 3; p--) k_lusgs<T, NV, true><<<gc, 128, 0, st>>>(A, p);
     } else {
       if (upper && I_.lu_version == 4 && I_.lu_fused) return;  // ran with the lower sweep's launch
-      if (!upper) cudaMemsetAsync(L_.counter, 0, 2 * sizeof(int), st);
-      if (I_.lu_version != 5) cudaMemsetAsync(L_.progress, 0, sizeof(int) * L_.ntiles, st);
+      if (I_.lu_version != 5) {  // version 5 leaves its counter at 0 and keeps no progress
+        if (!upper) cudaMemsetAsync(L_.counter, 0, 2 * sizeof(int), st);
+        cudaMemsetAsync(L_.progress, 0, sizeof(int) * L_.ntiles, st);
+      }
       if (I_.lu_version == 5) {
         if (I_.lu_tc == 64) {
           if (!upper) k_lusgs_wave5<T, NV, false, 64><<<I_.lu_grid, lu5_threads<64>(), lu5_smem<T, NV, false, 64>(), st>>>(A, L_);
@@ -302,17 +304,12 @@ class RunnerT : public Runner {
       if (fresh && I_.xr_cells > 0) k_halo_unpack<T, NV><<<grid_of(I_.xr_cells), 256, 0, st>>>(A, I_.xr_sub, I_.xr_pre, I_.nxr, I_.xr_cells, I_.xrecv);
     }
     k_corner<T, NV><<<dim3(A.nblk, 8), 256, 0, st>>>(A);
-    k_corner_vtx<T, NV><<<grid_of((long long)A.nblk * NV * 8, 128), 128, 0, st>>>(A);
   }
 
   void limit(cudaStream_t st) {
     const Arena<T>& A = A_;
-    k_limit_fix<T><<<grid_of(A.tot_cell), 256, 0, st>>>(A);
-    if (NV == 6) {  // order: the cells above LSAmax first, then the clamp of all others
-      k_sa_limit_check<T><<<grid_of(A.tot_cell), 256, 0, st>>>(A);
-      k_sa_limit_serial<T><<<A.nblk, SAL_THREADS, 0, st>>>(A);
-      k_sa_limit_par<T><<<grid_of(A.tot_cell), 256, 0, st>>>(A);
-    }
+    if (NV == 6) k_sa_limit_serial<T><<<A.nblk, SAL_THREADS, 0, st>>>(A);  // the cells above LSAmax, then the clamp of all others
+    k_limit_fix<T, NV == 6><<<grid_of(A.tot_cell), 256, 0, st>>>(A);
   }
 
   void step(cudaStream_t st, cudaEvent_t* ev = nullptr) override {
@@ -385,10 +382,10 @@ class RunnerT : public Runner {
       else if (I_.turb == 3 && NV == 7) res += 11;
     }
     int lu = I_.lu_planes ? 2 * (I_.max_plane - 2) : (I_.lu_version == 4 && I_.lu_fused ? 1 : 2);
-    int upd = 1 + 1 + (NV == 6 ? 3 : 0);
+    int upd = 1 + 1 + (NV == 6 ? 1 : 0);
     int nbc = 0;
     for (int r = 0; r < I_.nround; r++) nbc += I_.bc_rounds[3 * r + 2] > 0;
-    int bch = nbc + 2 + (A_.tot_halo > 0 ? (I_.nhlevel ? 2 * I_.nhlevel : 1) : 0) + (I_.xs_cells > 0) + (I_.xr_cells > 0);
+    int bch = nbc + 1 + (A_.tot_halo > 0 ? (I_.nhlevel ? 2 * I_.nhlevel : 1) : 0) + (I_.xs_cells > 0) + (I_.xr_cells > 0);
     int n;
     if (I_.time_method == -1) return res + 1 + lu + upd + bch;  // one dual-time inner iteration
     if (I_.time_method == 0) n = res + lu + upd + bch;

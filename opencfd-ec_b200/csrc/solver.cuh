@@ -1466,6 +1466,7 @@ __global__ void k_update(Arena<T> A) {
       double p1 = (Un[4] - 0.5 * d1 * (u1 * u1 + v1 * v1 + w1 * w1)) * (s.gamma - 1.0);
       A.DU[g] = d1; A.DU[tc + g] = u1; A.DU[2 * tc + g] = v1; A.DU[3 * tc + g] = w1; A.DU[4 * tc + g] = p1;
       if (lim_bad(s, d1, u1, v1, w1, p1)) atomicAdd(&A.flags[A.nblk + b], 1);
+      if (NV == 6 && Un[5] > s.lsamax) A.flags[2 * A.nblk + b] = 1;  // k_sa_limit_serial has work in this block
     }
   }
 }
@@ -1513,15 +1514,23 @@ __global__ void k_dual_init(Arena<T> A) {
   OCFD_GRID_STRIDE(g, n) { A.Un[g] = A.U[g]; A.Un1[g] = A.U[g]; }
 }
 
-// neighbour-average repair of bad cells (sub_limitflow.f90:84-150); DU planes 0..4 hold d,u,v,w,p
-template <class T>
+// neighbour-average repair of bad cells (sub_limitflow.f90:84-150); DU planes 0..4 hold d,u,v,w,p.
+// SA: also the clamp of the SA variable to SAmin that ends limit_flow_SA (below): the repair does not
+// touch it
+template <class T, bool SA>
 __global__ void k_limit_fix(Arena<T> A) {
   const long long tb = A.tot_box, tc = A.tot_cell;
   OCFD_GRID_STRIDE(g, tc) {
     int b = find_blk_h(A.pre_cell, A.hint_cell, A.nblk, g);
-    if (A.flags[A.nblk + b] == 0) continue;
     const BlkD& B = A.blk[b];
     const SolveP& s = A.sp[B.solve];
+    if (SA && s.limit_flow == 1) {
+      int i, j, k;
+      dec_cell(B, g - B.ocell, i, j, k);
+      const long long c = 5 * tb + bix(B, i, j, k);
+      if (A.U[c] < 1.e-8) A.U[c] = 1.e-8;
+    }
+    if (A.flags[A.nblk + b] == 0) continue;
     const double *d1 = A.DU, *u1 = A.DU + tc, *v1 = A.DU + 2 * tc, *w1 = A.DU + 3 * tc, *p1 = A.DU + 4 * tc;
     if (!lim_bad(s, d1[g], u1[g], v1[g], w1[g], p1[g])) continue;
     int i, j, k;
@@ -1565,31 +1574,8 @@ __global__ void k_limit_fix(Arena<T> A) {
 // what it holds in the array before the clamp pass, whether it was above LSAmax (replaced by an
 // average in [SAmin, LSAmax]) or not.  That makes the order matter only among the cells above
 // LSAmax, which k_sa_limit_serial visits in order (reading earlier neighbours as max(v, SAmin) and
-// later ones as they are); k_sa_limit_par then clamps every other cell to SAmin in parallel.
-template <class T>
-__global__ void k_sa_limit_check(Arena<T> A) {
-  const long long tb = A.tot_box;
-  OCFD_GRID_STRIDE(g, A.tot_cell) {
-    int b = find_blk_h(A.pre_cell, A.hint_cell, A.nblk, g);
-    const BlkD& B = A.blk[b];
-    int i, j, k;
-    dec_cell(B, g - B.ocell, i, j, k);
-    if (A.sp[B.solve].limit_flow == 1 && A.U[5 * tb + bix(B, i, j, k)] > A.sp[B.solve].lsamax) A.flags[2 * A.nblk + b] = 1;
-  }
-}
-template <class T>
-__global__ void k_sa_limit_par(Arena<T> A) {
-  const long long tb = A.tot_box;
-  OCFD_GRID_STRIDE(g, A.tot_cell) {
-    int b = find_blk_h(A.pre_cell, A.hint_cell, A.nblk, g);
-    const BlkD& B = A.blk[b];
-    if (A.sp[B.solve].limit_flow != 1) continue;
-    int i, j, k;
-    dec_cell(B, g - B.ocell, i, j, k);
-    long long c = 5 * tb + bix(B, i, j, k);
-    if (A.U[c] < 1.e-8) A.U[c] = 1.e-8;
-  }
-}
+// later ones as they are); k_limit_fix then clamps every other cell to SAmin in parallel, and k_update
+// has flagged the blocks that hold a cell above LSAmax.
 // one CTA per block with a cell above LSAmax: the block is scanned in chunks of SAL_CHUNK cells in
 // the reference's order (warp ballots find the chunk's cells above LSAmax), and thread 0 replaces
 // those cells, in order, by the average of their neighbours
@@ -1654,13 +1640,15 @@ __global__ void __launch_bounds__(SAL_THREADS) k_sa_limit_serial(Arena<T> A) {
   }
 }
 
-// force_vt_kw (sub_time_advance.f90:27-61)
+// force_vt_kw (sub_time_advance.f90:27-61); for NV = 6 with the flow limiter on it has nothing to do
+// (limit_flow_SA left every interior value at 1e-8 or more), so blocks of such solves are skipped
 template <class T, int NV>
 __global__ void k_vtkw(Arena<T> A) {
   const long long tb = A.tot_box;
   OCFD_GRID_STRIDE(g, A.tot_cell) {
     int b = find_blk_h(A.pre_cell, A.hint_cell, A.nblk, g);
     const BlkD& B = A.blk[b];
+    if (NV == 6 && A.sp[B.solve].limit_flow == 1) continue;
     int i, j, k;
     dec_cell(B, g - B.ocell, i, j, k);
     long long c = bix(B, i, j, k);
@@ -1922,7 +1910,8 @@ __global__ void k_halo_unpack(Arena<T> A, const SubD* sub, const long long* pre,
   }
 }
 
-// edge and vertex ghosts by averaging (get_U_conner, sub_update_buffer_mpi.f90:515-549)
+// edge and vertex ghosts by averaging (get_U_conner, sub_update_buffer_mpi.f90:515-549), in one
+// launch: a vertex evaluates the three edge values it averages itself
 template <class T, int NV>
 __global__ void k_corner(Arena<T> A) {  // edges: grid (blocks, CTAs per block)
   const int b = blockIdx.x;
@@ -1960,28 +1949,16 @@ __global__ void k_corner(Arena<T> A) {  // edges: grid (blocks, CTAs per block)
       else u(m, i, ny, nz) = (u(m, i, ny - 1, nz) + u(m, i, ny, nz - 1)) * 0.5;
     }
   }
+  if (blockIdx.y == 0)
+    for (int r = threadIdx.x; r < NV * 8; r += blockDim.x) {  // the 8 vertices
+      const int m = r % NV, v = r / NV;
+      const int ia = (v & 1) ? nx : 0, ja = (v & 2) ? ny : 0, kz = (v & 4) ? nz : 0;
+      const int ib = (v & 1) ? nx - 1 : 1, jb = (v & 2) ? ny - 1 : 1, kb = (v & 4) ? nz - 1 : 1;
+      const double fi = u(m, ia, jb, kb), fj = u(m, ib, ja, kb), fk = u(m, ib, jb, kz);  // face ghosts
+      const double ei = (fk + fj) * 0.5, ej = (fk + fi) * 0.5, ek = (fj + fi) * 0.5;     // edge ghosts along i, j, k
+      u(m, ia, ja, kz) = (2.0 * (ei + ej + ek) - (fk + fj + fi)) / 3.0;
+    }
 }
-// the 8 vertices of every block from the edge values (after k_corner)
-template <class T, int NV>
-__global__ void k_corner_vtx(Arena<T> A) {
-  const long long tb = A.tot_box;
-  const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= (long long)A.nblk * NV * 8) return;
-  const int b = (int)(g / (NV * 8));
-  const BlkD& B = A.blk[b];
-  if (A.only_solve >= 0 && B.solve != A.only_solve) return;
-  const int nx = B.nx, ny = B.ny, nz = B.nz;
-  double* U = A.U;
-  auto u = [&](int m, int i, int j, int k) -> double& { return U[m * tb + bix(B, i, j, k)]; };
-  {
-    const int r = (int)(g % (NV * 8));
-    int m = r % NV, v = r / NV;
-    int ia = (v & 1) ? nx : 0, ja = (v & 2) ? ny : 0, kz = (v & 4) ? nz : 0;
-    int ib = (v & 1) ? nx - 1 : 1, jb = (v & 2) ? ny - 1 : 1, kb = (v & 4) ? nz - 1 : 1;
-    u(m, ia, ja, kz) = (2.0 * (u(m, ib, ja, kz) + u(m, ia, jb, kz) + u(m, ia, ja, kb)) - (u(m, ib, jb, kz) + u(m, ib, ja, kb) + u(m, ia, jb, kb))) / 3.0;
-  }
-}
-
 // ============================================================================================
 // residual norms (comput_max_Res_onemesh, sub_time_advance.f90:330-380): FP64, fixed chunks and
 // a fixed reduction tree, so the result is deterministic
