@@ -1097,7 +1097,7 @@ static int create_impl(const ocfd_params* ps, int nsolve, const int* nblk_s, con
   if (h->prec == OCFD_PREC_MIXED) fill_arena<float>(h, h->A32, h->d_Mf, h->d_volf, h->d_dtmf, h->d_dwf);
   else fill_arena<double>(h, h->A64, h->d_Md, h->d_vold, h->d_dtmd, h->d_dwd);
   // LU-SGS kernel: version 5 on 32-column tiles, the fastest form on every configuration (config 2:
-  // 0.51 ms a sweep against 0.69 of the best of versions 3 and 4, its 64-column form 0.82; see
+  // 0.49 ms a sweep against 0.69 of the best of versions 3 and 4, its 64-column form 0.82; see
   // lusgs5.cuh).  OCFD_LU_TC fixes the tile width, OCFD_LU_V3 / V4 / V5 the version (OCFD_LU_V2
   // both); versions 3 and 4 are timed against each other where the switches leave a choice, and
   // OCFD_NO_AUTOTUNE takes the first of them.  OCFD_LU_ONE_LAUNCH puts version 4's one-launch form

@@ -43,15 +43,18 @@
 // of lusgs.cuh: tiles are handed out in topological order to resident CTAs.
 //
 // Measured (B200, ms lower + upper sweep, the best of versions 3 and 4 -> this): config 2 (2.09 M
-// cells, 8 blocks) FP64 0.690 + 0.669 -> 0.513 + 0.505, mixed 0.623 + 0.664 -> 0.436 + 0.437; 64
-// airfoils mixed 0.742 + 0.704 -> 0.472 + 0.442; wing-body (7.8 M cells, SST) mixed 1.62 + 1.65 -> 1.31
-// + 1.31; one 129 x 33 airfoil FP64 0.194 -> 0.115 a sweep, the 129 x 65 x 17 channel 0.33 -> 0.16.  A
-// step takes about 1,300 cycles: the D warps' shared-memory reads (123 of 8 bytes a thread and step, the
-// burst after the barrier) and L's copies share the SM's load path, about 700 cycles a step together,
-// beside a chain of about 400.  Tried on top and slower: step counters with acquire loads in place of the
-// mbarriers (+3 %), DU shared between the D warps by variables with a second barrier (FP64 +15 %, mixed
-// even), 64-column tiles (+60 %), face geometry and state loaded by the D and P warps themselves into
-// registers (+20 to 40 %).
+// cells, 8 blocks) FP64 0.690 + 0.669 -> 0.491 + 0.493, mixed 0.623 + 0.664 -> 0.426 + 0.430; 64
+// airfoils mixed 0.742 + 0.704 -> 0.459 + 0.435; wing-body (7.8 M cells, SST) mixed 1.62 + 1.65 -> 1.30
+// + 1.29; one 129 x 33 airfoil FP64 0.194 -> 0.110 a sweep, the 129 x 65 x 17 channel 0.33 -> 0.16.  A
+// step takes about 1,300 cycles: a D warp's ~320 instructions at four to five cycles each (a chain of
+// dependent FP64 operations and shared-memory reads), beside the SM's load path at about half of its
+// rate (ncu on the channel, a step of a tile: 1,566 warp instructions of all roles, 666 wavefronts, of
+// which 263 shared-memory loads, 198 of L's copies and 69 stores).  Tried on top and slower: step
+// counters with acquire loads in place of the mbarriers (+3 %), DU shared between the D warps by
+// variables with a second barrier (FP64 +15 %, mixed even), next step's mbarriers probed a step ahead
+// (even), two CTAs per SM at 168 registers with one P and one L warp (config 2 FP64 +90 %: the single L
+// warp bounds it), 64-column tiles (+60 %), face geometry and state loaded by the D and P warps
+// themselves into registers (+20 to 40 %).
 #pragma once
 #include "lusgs.cuh"
 
@@ -119,6 +122,12 @@ __device__ __forceinline__ void cp_elem(unsigned dst, const X* src) {
 }
 __device__ __forceinline__ void cp_arrive(unsigned a) { asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(a) : "memory"); }
 
+// N values of one term
+template <int N>
+struct alignas(8 * N) Lu5Vec {
+  double v[N];
+};
+
 // ---- shared memory (byte offsets) -------------------------------------------------------------
 // Input rows: one row of TC cells per stream and step, 2 WB rows per stream (two blocks).  The row
 // pitch is TC + 2 doubles or TC + 4 floats: the copies of a request (32 / WB columns x WB steps, a
@@ -137,7 +146,10 @@ struct Lu5Smem {
   static constexpr int SLOT0 = S + 3 * ROWS * PT;
   static constexpr int NA = sizeof(T) == 8 ? (NV == 6 ? 4 : 2) : (NV == 6 ? 2 : 1);  // diagonal: (value and) reciprocal, SA's own
   static constexpr int AS = 2 * TC + 2;  // the place behind the edges stays zero
-  static constexpr int ACC = 0, AL = ACC + 3 * NV * AS * 8, Q = AL + NA * TC * 8;  // Q: 1/rho, E - kinetic energy
+  // a term's values lie in pairs of variables (one 16-byte access) for NV = 6: sweep -4 % on the SA
+  // airfoil and wing; padding an odd NV costs more than it saves (SST airfoil 0.242 -> 0.270 ms)
+  static constexpr int VP = NV % 2 == 0 ? 2 : 1, NP2 = NV / VP, VB = 8 * VP;
+  static constexpr int ACC = 0, AL = ACC + 3 * NP2 * AS * VB, Q = AL + NA * TC * 8;  // Q: 1/rho, E - kinetic energy
   static constexpr int SU = Q + 2 * TC * (int)sizeof(T);                         // mixed form: the state in FP32
   static constexpr int SLOT = (SU + (sizeof(T) == 4 ? NV * TC * 4 : 0) + 15) / 16 * 16;
   static constexpr int BYTES = SLOT0 + SLOTS * SLOT;
@@ -152,6 +164,8 @@ template <class T, int NV, bool UPPER, int TC>
 __global__ void __launch_bounds__(7 * TC + 32, 1) k_lusgs_wave5(Arena<T> A, LuArgs L) {
   using SM = Lu5Smem<T, NV, UPPER, TC>;
   using RT = typename SM::RT;
+  using VT = Lu5Vec<SM::VP>;
+  using T2 = typename std::conditional<sizeof(T) == 8, double2, float2>::type;
   constexpr int SLOTS = SM::SLOTS, WB = SM::WB, RW = TC / 32, NA = SM::NA, PB = SM::PB, PT = SM::PT, ROWS = SM::ROWS;
   constexpr bool FP64 = sizeof(T) == 8;
   constexpr int AS5 = NV == 6 ? 2 : 0;  // the SA variable's own diagonal (FP64 form: value, reciprocal)
@@ -173,8 +187,8 @@ __global__ void __launch_bounds__(7 * TC + 32, 1) k_lusgs_wave5(Arena<T> A, LuAr
     for (int q = 0; q < SLOTS; q++) { mb_init(fullP + 8 * q, RW); mb_init(fullE + 8 * q, 1); mb_init(empty0 + 8 * q, 3 * RW); }
     for (int q = 0; q < 2; q++) { mb_init(fullR + 8 * q, 2 * TC); mb_init(emptyR + 8 * q, 3 * RW); }
   }
-  for (int q = tid; q < SLOTS * 3 * NV; q += lu5_threads<TC>())  // the zero places
-    reinterpret_cast<double*>(s_dyn + SM::SLOT0 + q / (3 * NV) * SM::SLOT + SM::ACC)[(q % (3 * NV)) * SM::AS + 2 * TC] = 0.0;
+  for (int q = tid; q < SLOTS * 3 * SM::NP2; q += lu5_threads<TC>())  // the zero places
+    reinterpret_cast<VT*>(s_dyn + SM::SLOT0 + q / (3 * SM::NP2) * SM::SLOT + SM::ACC)[(q % (3 * SM::NP2)) * SM::AS + 2 * TC] = VT{};
   // steps and row blocks this CTA has done (the same in every role): slot it % SLOTS, round
   // it / SLOTS; block buffer ib % 2, round ib / 2
   unsigned it = 0, ib = 0;
@@ -210,9 +224,9 @@ __global__ void __launch_bounds__(7 * TC + 32, 1) k_lusgs_wave5(Arena<T> A, LuAr
       const bool has_j = UPPER ? j != nym : j != 1, has_k = UPPER ? k != nzm : k != 1;  // upstream neighbours
       // places of the upstream terms: the own column's, its neighbours' (or the upstream edges' behind
       // them), or the zero place where there is no neighbour
-      const int a_i = c * 8, a_z = 2 * TC * 8;
-      const int a_j = (NV * SM::AS + (!has_j ? 2 * TC : (lj > 0 ? c - 1 : TC + c + TJ - 1))) * 8;
-      const int a_k = (2 * NV * SM::AS + (!has_k ? 2 * TC : (lk > 0 ? c - TJ : TC + TC - TJ + lj))) * 8;
+      const int a_i = c * SM::VB, a_z = 2 * TC * SM::VB;
+      const int a_j = (SM::NP2 * SM::AS + (!has_j ? 2 * TC : (lj > 0 ? c - 1 : TC + c + TJ - 1))) * SM::VB;
+      const int a_k = (2 * SM::NP2 * SM::AS + (!has_k ? 2 * TC : (lk > 0 ? c - TJ : TC + TC - TJ + lj))) * SM::VB;
       // does this column's term leave the tile?  Edge words: j edge [step][m][lk], then k edge [step][m][lj]
       const bool out = d == 1 ? (lj == TJ - 1 && (UPPER ? J > 0 : J < nJ - 1)) : (d == 2 && lk == TK - 1 && (UPPER ? K > 0 : K < nK - 1));
       const int ow = d == 1 ? TK : TJ;
@@ -241,10 +255,19 @@ __global__ void __launch_bounds__(7 * TC + 32, 1) k_lusgs_wave5(Arena<T> A, LuAr
         x.g[3] = (T)(UPPER ? -0.5 : 0.5) * *reinterpret_cast<const T*>(rt + SM::S + d * ROWS * PT);
         x.g[4] = (T)0.5 * (T)(w * (double)*reinterpret_cast<const T*>(rt + SM::LC + d * ROWS * PT));
         x.g[5] = *reinterpret_cast<const T*>(rt + SM::LV + d * ROWS * PT);
+        if constexpr (NA == 1) {
+          x.al[0] = reinterpret_cast<const double*>(sl + SM::AL)[c];
+        } else {
 #pragma unroll
-        for (int m = 0; m < NA; m++) x.al[m] = reinterpret_cast<const double*>(sl + SM::AL)[m * TC + c];
-        x.r0 = reinterpret_cast<const T*>(sl + SM::Q)[c];
-        x.ei = reinterpret_cast<const T*>(sl + SM::Q)[TC + c];
+          for (int m = 0; m < NA / 2; m++) {
+            const double2 p = reinterpret_cast<const double2*>(sl + SM::AL)[m * TC + c];
+            x.al[2 * m] = p.x;
+            x.al[2 * m + 1] = p.y;
+          }
+        }
+        const T2 q = reinterpret_cast<const T2*>(sl + SM::Q)[c];
+        x.r0 = q.x;
+        x.ei = q.y;
       };
       // F(U).n of the old state (plain: by plain division); true: operands div_by does not cover
       auto old_flux = [&](const Cell& x, T* F, bool plain) -> bool {
@@ -333,11 +356,15 @@ __global__ void __launch_bounds__(7 * TC + 32, 1) k_lusgs_wave5(Arena<T> A, LuAr
             const unsigned char* const acc = sl + SM::ACC;
             const int ai = t - lj - lk > 0 ? a_i : a_z;
 #pragma unroll
-            for (int m = 0; m < NV; m++) {
-              const double a0 = *reinterpret_cast<const double*>(acc + ai + m * SM::AS * 8);
-              const double a1 = *reinterpret_cast<const double*>(acc + a_j + m * SM::AS * 8);
-              const double a2 = *reinterpret_cast<const double*>(acc + a_k + m * SM::AS * 8);
-              xs[m] = UPPER ? a0 + a1 + a2 : (double)xc.R[m] + a0 + a1 + a2;
+            for (int p = 0; p < SM::NP2; p++) {
+              const VT b0 = *reinterpret_cast<const VT*>(acc + ai + p * SM::AS * SM::VB);
+              const VT b1 = *reinterpret_cast<const VT*>(acc + a_j + p * SM::AS * SM::VB);
+              const VT b2 = *reinterpret_cast<const VT*>(acc + a_k + p * SM::AS * SM::VB);
+#pragma unroll
+              for (int e = 0; e < SM::VP; e++) {
+                const int m = SM::VP * p + e;
+                xs[m] = UPPER ? b0.v[e] + b1.v[e] + b2.v[e] : (double)xc.R[m] + b0.v[e] + b1.v[e] + b2.v[e];
+              }
             }
           }
           take(xn, ns, row_of(t + 1));
@@ -349,9 +376,14 @@ __global__ void __launch_bounds__(7 * TC + 32, 1) k_lusgs_wave5(Arena<T> A, LuAr
             cell(xc, F[u], xs, DU, v, true);
             old_flux(xn, F[1 - u], true);
           }
-          double* const nacc = reinterpret_cast<double*>(ns + SM::ACC) + d * NV * SM::AS + c;
+          VT* const nacc = reinterpret_cast<VT*>(ns + SM::ACC) + d * SM::NP2 * SM::AS + c;
 #pragma unroll
-          for (int m = 0; m < NV; m++) nacc[m * SM::AS] = v[m];
+          for (int p = 0; p < SM::NP2; p++) {
+            VT x2;
+#pragma unroll
+            for (int e = 0; e < SM::VP; e++) x2.v[e] = v[SM::VP * p + e];
+            nacc[p * SM::AS] = x2;
+          }
           if (out && on) {
 #pragma unroll
             for (int m = 0; m < NV; m++) st_word(eout + t * (NV * ow) + m * ow, __double_as_longlong(v[m]));
@@ -420,18 +452,21 @@ __global__ void __launch_bounds__(7 * TC + 32, 1) k_lusgs_wave5(Arena<T> A, LuAr
         double ra = rcp_rn(al), ras = NV == 6 ? rcp_rn(als) : 0.0;
         if (bad_den(al) || (NV == 6 && bad_den(als))) { ra = 1.0 / al; ras = 1.0 / als; }
         mb_wait(empty0 + 8 * (n % SLOTS), (n / SLOTS + 1) & 1, L.err);  // the slot's last readers are done
-        double* const pa = reinterpret_cast<double*>(sl + SM::AL) + c;
-        if (FP64) {
-          pa[0] = al; pa[TC] = ra;
-          if (NV == 6) { pa[AS5 * TC] = als; pa[(AS5 + 1) * TC] = ras; }
+        if constexpr (NA == 1) {
+          reinterpret_cast<double*>(sl + SM::AL)[c] = ra;
         } else {
-          pa[0] = ra;
-          if (NV == 6) pa[(NA - 1) * TC] = ras;
+          double2* const pa = reinterpret_cast<double2*>(sl + SM::AL) + c;
+          pa[0] = FP64 ? make_double2(al, ra) : make_double2(ra, ras);
+          if (NA == 4) pa[TC] = make_double2(als, ras);
+        }
+        T2 q2;
+        q2.x = r0;
+        q2.y = ei;
+        reinterpret_cast<T2*>(sl + SM::Q)[c] = q2;
+        if (!FP64) {
 #pragma unroll
           for (int m = 0; m < NV; m++) reinterpret_cast<T*>(sl + SM::SU)[m * TC + c] = U[m];
         }
-        reinterpret_cast<T*>(sl + SM::Q)[c] = r0;
-        reinterpret_cast<T*>(sl + SM::Q)[TC + c] = ei;
         __syncwarp();
         if (lane == 0) mb_arrive(fullP + 8 * (n % SLOTS));
       }
@@ -527,13 +562,13 @@ __global__ void __launch_bounds__(7 * TC + 32, 1) k_lusgs_wave5(Arena<T> A, LuAr
           const int m = x / TK, ek = x % TK, kk = UPPER ? tl.k0 + TK - 1 - ek : tl.k0 + ek;
           if (up_j && kk >= 1 && kk <= nzm) {
             src[e] = L.edge + L.edge_off[step_j] + ((long long)(TJ - 1) * NV + m) * TK + ek;
-            stride[e] = NV * TK; lo[e] = ek; dst[e] = (1 * NV + m) * SM::AS + TC + ek * TJ + TJ - 1;
+            stride[e] = NV * TK; lo[e] = ek; dst[e] = ((SM::NP2 + m / SM::VP) * SM::AS + TC + ek * TJ + TJ - 1) * SM::VP + m % SM::VP;
           }
         } else if (x < NV * (TJ + TK)) {  // k edge
           const int m = (x - NV * TK) / TJ, ej = (x - NV * TK) % TJ, jj = UPPER ? tl.j0 + TJ - 1 - ej : tl.j0 + ej;
           if (up_k && jj >= 1 && jj <= nym) {
             src[e] = L.edge + L.edge_off[step_k] + (long long)nsteps * NV * TK + ((long long)(TK - 1) * NV + m) * TJ + ej;
-            stride[e] = NV * TJ; lo[e] = ej; dst[e] = (2 * NV + m) * SM::AS + TC + TC - TJ + ej;
+            stride[e] = NV * TJ; lo[e] = ej; dst[e] = ((2 * SM::NP2 + m / SM::VP) * SM::AS + TC + TC - TJ + ej) * SM::VP + m % SM::VP;
           }
         }
       }
