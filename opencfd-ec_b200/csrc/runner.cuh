@@ -116,7 +116,6 @@ class RunnerT : public Runner {
     }
     if (fork) inviscid(is);
     if (I_.viscous) {
-      k_mu<T><<<grid_of(tc), 256, 0, cs>>>(A);
       if (I_.turb == 2 && NV == 6) {
         k_sa_pre<T><<<grid_of(A.tot_r1), 256, 0, cs>>>(A);
         if (I_.sa_fused) {
@@ -141,6 +140,7 @@ class RunnerT : public Runner {
         k_sst_res<T><<<grid_of(tc), 256, 0, cs>>>(A);
         k_mu_finish<T, 1><<<grid_of(A.tot_r1), 256, 0, cs>>>(A);
       } else {
+        k_mu<T><<<grid_of(tc), 256, 0, cs>>>(A);
         cudaMemsetAsync(A.mut, 0, sizeof(T) * tb, cs);
       }
       k_amut<T><<<grid_of(A.tot_subcell), 256, 0, cs>>>(A);
@@ -377,9 +377,10 @@ class RunnerT : public Runner {
     else if (I_.res_fused == 3) res += 4 + 1;
     else res += 4 + vis + 1 + (st2_ && sizeof(T) == 8 ? 1 : 0);  // forked FP64: k_cell_dt beside the viscous fluxes
     if (I_.viscous) {
-      res += 1 + 1;  // mu, amut
+      res += 1;  // amut
       if (I_.turb == 2 && NV == 6) res += I_.sa_fused ? 3 : 6;  // sa_pre, (tile | 3 fluxes + res), mu_finish
       else if (I_.turb == 3 && NV == 7) res += 11;
+      else res += 1;  // mu
     }
     int lu = I_.lu_planes ? 2 * (I_.max_plane - 2) : (I_.lu_version == 4 && I_.lu_fused ? 1 : 2);
     int upd = 1 + 1 + (NV == 6 ? 1 : 0);

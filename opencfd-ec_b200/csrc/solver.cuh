@@ -113,19 +113,31 @@ __global__ void k_prim(Arena<T> A) {
   }
 }
 
-// get_viscous (sub_Residual.f90:1355-1383): Sutherland mu on the interior + the 6 face ghost
-// layers (edge/corner ghosts keep their previous values, as in the reference)
+// Sutherland mu of an interior cell (get_viscous, sub_Residual.f90:1355-1383)
+template <class T>
+__device__ __forceinline__ T sutherland(const Arena<T>& A, const BlkD& B, const SolveP& s, int i, int j, int k) {
+  const double Tt = (double)A.P[P_T * A.tot_box + bix(B, i, j, k)];
+  return T(1.0 / s.re * (1.0 + s.tsb) * sqrt(cube(Tt)) / (s.tsb + Tt));
+}
+// the same on the 0..n layer: a face ghost takes its interior cell's value, edge and corner ghosts keep
+// their previous ones (as in the reference).  The turbulence models' first kernels evaluate it
+// themselves (a launch and a pass over mu less than k_mu before them)
+template <class T>
+__device__ __forceinline__ T mu_r1(const Arena<T>& A, const BlkD& B, const SolveP& s, int i, int j, int k, long long g) {
+  const int ic = min(max(i, 1), B.nx - 1), jc = min(max(j, 1), B.ny - 1), kc = min(max(k, 1), B.nz - 1);
+  return (ic != i) + (jc != j) + (kc != k) <= 1 ? sutherland(A, B, s, ic, jc, kc) : A.mu[g];
+}
+
+// mu of a laminar case: interior + the 6 face ghost layers
 template <class T>
 __global__ void k_mu(Arena<T> A) {
-  const long long tb = A.tot_box;
   OCFD_GRID_STRIDE(g, A.tot_cell) {
     int b = find_blk_h(A.pre_cell, A.hint_cell, A.nblk, g);
     const BlkD& B = A.blk[b];
     const SolveP& s = A.sp[B.solve];
     int i, j, k;
     dec_cell(B, g - B.ocell, i, j, k);
-    double Tt = (double)A.P[P_T * tb + bix(B, i, j, k)];
-    T mu = T(1.0 / s.re * (1.0 + s.tsb) * sqrt(cube(Tt)) / (s.tsb + Tt));
+    const T mu = sutherland(A, B, s, i, j, k);
     A.mu[bix(B, i, j, k)] = mu;
     if (i == 1) A.mu[bix(B, 0, j, k)] = mu;
     if (i == B.nx - 1) A.mu[bix(B, B.nx, j, k)] = mu;
@@ -158,7 +170,7 @@ __global__ void k_sa_pre(Arena<T> A) {
     dec_r1(B, r - B.or1, i, j, k);
     const long long g = bix(B, i, j, k);
     const SolveP& s = A.sp[B.solve];
-    T mu = T((double)A.mu[g] * s.re);
+    T mu = T((double)mu_r1(A, B, s, i, j, k, g) * s.re);
     T vt = T(clamp0(A.U[5 * tb + g]));
     T d = A.P[P_D * tb + g];
     A.mu[g] = mu;  // after the loads: a store before them would hold them back
@@ -394,7 +406,7 @@ __global__ void k_sst_pre(Arena<T> A) {
     dec_r1(B, r - B.or1, i, j, k);
     const long long g = bix(B, i, j, k);
     const SolveP& s = A.sp[B.solve];
-    const T mu = T((double)A.mu[g] * s.re);
+    const T mu = T((double)mu_r1(A, B, s, i, j, k, g) * s.re);
     const double d = A.U[g], u5 = A.U[5 * tb + g], u6 = A.U[6 * tb + g];  // loads before the stores
     A.mu[g] = mu;
     A.Kt[g] = T(clamp0(u5) / d);
