@@ -1913,35 +1913,45 @@ extern "C" int ocfd_array_shape(const ocfd_handle* h, int b, const char* name, i
   return OCFD_OK;
 }
 
-// copies the array in the requested Fortran bounds; variable-major planes are interleaved back
-// to the Fortran (m fastest) order
+// one array of a block into the requested Fortran bounds, cell-major with nv values per cell (m
+// fastest), as doubles: w0 x w1 x w2 cells from index lo, of a stored range n0 x n1 from index base_lo
+struct GatherD {
+  const void* base;
+  long long plane, off, n0, n1, cells;
+  int dbl, nv, base_lo, lo[3];
+  unsigned w0, w1;
+};
+__global__ void k_gather_array(GatherD d, double* out) {
+  for (long long l = (long long)blockIdx.x * blockDim.x + threadIdx.x; l < d.cells; l += (long long)gridDim.x * blockDim.x) {
+    const unsigned u = (unsigned)l, t = u / d.w0;  // a block's ghost box holds fewer than 2^31 cells
+    const int i = (int)(u - t * d.w0) + d.lo[0], j = (int)(t % d.w1) + d.lo[1], k = (int)(t / d.w1) + d.lo[2];
+    const long long src = d.off + (i - d.base_lo) + d.n0 * ((j - d.base_lo) + d.n1 * (long long)(k - d.base_lo));
+    for (int m = 0; m < d.nv; m++)
+      out[l * d.nv + m] = d.dbl ? ((const double*)d.base)[m * d.plane + src] : (double)((const float*)d.base)[m * d.plane + src];
+  }
+}
+
+// copies the array in the requested Fortran bounds, interleaved on the device into the state's
+// staging area and read back in one transfer (a host loop over the values took most of the call: state in,
+// residual, 131,072 x 5 FP32 values out 2.13 -> 1.30 ms)
 extern "C" int ocfd_get_array(ocfd_handle* h, int b, const char* name, double* out) {
   if (!h || !name || !out || b < 0 || b >= h->nblk) return OCFD_ERR_ARG;
   ArrDesc d;
   if (!describe(h, b, name, d)) return OCFD_ERR_ARG;
   const BlkD& B = h->blk[b];
-  long long off, n0, n1, n2;
-  int base_lo;
-  if (d.space == 0) { off = B.obox; n0 = B.NX; n1 = B.NY; n2 = B.NZ; base_lo = -3; }
-  else if (d.space == 1) { off = B.oface; n0 = B.nx; n1 = B.ny; n2 = B.nz; base_lo = 1; }
-  else { off = B.ocell; n0 = B.nx - 1; n1 = B.ny - 1; n2 = B.nz - 1; base_lo = 1; }
-  long long cnt = n0 * n1 * n2;
-  size_t es = d.is_double ? 8 : 4;
-  std::vector<char> tmp(cnt * es * d.nv);
-  for (int m = 0; m < d.nv; m++) {
-    cudaError_t e = cudaMemcpy(&tmp[m * cnt * es], (const char*)d.base + (size_t)(m * d.plane + off) * es, cnt * es, cudaMemcpyDeviceToHost);
-    if (e != cudaSuccess) return cuda_fail(h, e, "get_array");
-  }
-  long long w0 = d.hi[0] - d.lo[0] + 1, w1 = d.hi[1] - d.lo[1] + 1;
-  for (int k = d.lo[2]; k <= d.hi[2]; k++)
-    for (int j = d.lo[1]; j <= d.hi[1]; j++)
-      for (int i = d.lo[0]; i <= d.hi[0]; i++) {
-        long long src = (i - base_lo) + n0 * ((j - base_lo) + n1 * (long long)(k - base_lo));
-        long long dst = (i - d.lo[0]) + w0 * ((j - d.lo[1]) + w1 * (long long)(k - d.lo[2]));
-        for (int m = 0; m < d.nv; m++) {
-          double v = d.is_double ? ((double*)tmp.data())[m * cnt + src] : (double)((float*)tmp.data())[m * cnt + src];
-          out[dst * d.nv + m] = v;
-        }
-      }
+  GatherD g;
+  g.base = d.base; g.dbl = d.is_double; g.nv = d.nv; g.plane = d.plane;
+  if (d.space == 0) { g.off = B.obox; g.n0 = B.NX; g.n1 = B.NY; g.base_lo = -3; }
+  else if (d.space == 1) { g.off = B.oface; g.n0 = B.nx; g.n1 = B.ny; g.base_lo = 1; }
+  else { g.off = B.ocell; g.n0 = B.nx - 1; g.n1 = B.ny - 1; g.base_lo = 1; }
+  for (int q = 0; q < 3; q++) g.lo[q] = d.lo[q];
+  g.w0 = (unsigned)(d.hi[0] - d.lo[0] + 1);
+  g.w1 = (unsigned)(d.hi[1] - d.lo[1] + 1);
+  g.cells = (long long)g.w0 * g.w1 * (d.hi[2] - d.lo[2] + 1);
+  k_gather_array<<<(int)std::min<long long>((g.cells + 255) / 256, 148 * 16), 256, 0, h->st>>>(g, h->d_stage);
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaMemcpyAsync(out, h->d_stage, sizeof(double) * g.nv * g.cells, cudaMemcpyDeviceToHost, h->st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(h->st);
+  if (e != cudaSuccess) return cuda_fail(h, e, "get_array");
   return OCFD_OK;
 }
