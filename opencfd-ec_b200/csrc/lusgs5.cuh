@@ -60,7 +60,9 @@
 
 namespace ocfd {
 
-constexpr int LU5_PACE = 300;  // ns between a loader warp's requests: keeps bursts off the load path (wing-body sweep 1.37 -> 1.31 ms)
+// ns between a loader warp's requests: keeps bursts off the load path (wing-body sweep 1.37 -> 1.31 ms).
+// Flat from 300 to 400 (257x97x86 FP64 step 2.60 ms); 150 gives 2.64 ms, 700 gives 2.68 ms.
+constexpr int LU5_PACE = 300;
 constexpr long long LU5_EMPTY = -1LL;  // the sentinel of an edge word
 
 // ---- division by a shared reciprocal -------------------------------------------------------
