@@ -672,10 +672,11 @@ __device__ __forceinline__ void inv_face(const Arena<T>& A, const BlkD& B, const
   long long c0 = bix(B, i - 4 * di, j - 4 * dj, k - 4 * dk);
   const long long st = DIR == 0 ? 1 : (DIR == 1 ? (long long)B.NX : (long long)B.NX * B.NY);
   T UL[5], UR[5];
-  // the FP64 WENO5 / MUSCL3 + Roe instantiations divide through reciprocals, without branches (the
-  // same bits): 57 divisions a WENO5 face, each a subroutine that kept the five variables from
+  // the FP64 WENO5 / MUSCL3 + Roe instantiations divide through reciprocals, without branches (the same
+  // bits but for the exceptions stated at rcp_near in physics.cuh): 57 divisions a WENO5 face, each a subroutine that kept the five variables from
   // overlapping (config 2 residual phase 1.74 -> 1.55 ms, step 2.87 -> 2.71 ms).  A face with operands
   // outside that division's range is evaluated again out of line
+  ExRange x;
   constexpr bool FAST = sizeof(T) == 8 && (ISCH == S_WENO5 || ISCH == S_MUSCL3) && IFLUX == F_ROE;
   if ((PRIM || s.recon == 0) && ISCH >= 0 && scheme == ISCH) {
 #pragma unroll
@@ -685,10 +686,10 @@ __device__ __forceinline__ void inv_face(const Arena<T>& A, const BlkD& B, const
 #pragma unroll
       for (int q = 0; q < 8; q++) u[q] = A.P[pl * tb + c0 + q * st];
       if constexpr (FAST && ISCH == S_WENO5) {
-        UL[m] = weno5_fast(u[1], u[2], u[3], u[4], u[5]);
-        UR[m] = weno5_fast(u[6], u[5], u[4], u[3], u[2]);
+        UL[m] = weno5_fast(u[1], u[2], u[3], u[4], u[5], x);
+        UR[m] = weno5_fast(u[6], u[5], u[4], u[3], u[2], x);
       } else if constexpr (FAST) {
-        muscl3_fast(u, UL[m], UR[m]);
+        muscl3_fast(u, UL[m], UR[m], x);
       } else {
         scheme_LR(u, ISCH < 0 ? 0 : ISCH, UL[m], UR[m]);
       }
@@ -775,7 +776,6 @@ __device__ __forceinline__ void inv_face(const Arena<T>& A, const BlkD& B, const
   };
   rotate();
   if constexpr (FAST) {
-    ExRange x;
     flux_roe_fast(QL, QR, F0, s.gamma, x);
     if (x.bad()) {
       T Fp[5];
