@@ -396,10 +396,14 @@ static void select_lu(ocfd_handle* h, int v, int ver) {
   else h->run.reset(make_runner_fp64(h->A64, h->info));
 }
 
-// version 5: every edge word empty again (after a timed-out wait, whose tile left words unread)
+// version 5: every edge word empty (at creation, and after a timed-out wait, whose tile left words unread)
+__global__ void k_empty_edges(long long* w, long long n) {
+  for (long long l = (long long)blockIdx.x * blockDim.x + threadIdx.x; l < n; l += (long long)gridDim.x * blockDim.x) w[l] = LU5_EMPTY;
+}
 static void reset_lu_edges(ocfd_handle* h) {
   for (int v = 0; v < 2; v++)
-    if (h->lu_edge_words[v] > 0) cudaMemsetAsync(h->lu_var[v].edge, 0xFF, (size_t)h->lu_edge_words[v] * sizeof(long long), h->st);
+    if (const long long n = h->lu_edge_words[v])
+      k_empty_edges<<<(int)std::min<long long>((n + 255) / 256, 148 * 16), 256, 0, h->st>>>(h->lu_var[v].edge, n);
 }
 
 // LU-SGS autotuner: each candidate (tile table v, kernel version ver) sweeps the freshly
@@ -1022,7 +1026,7 @@ static int create_impl(const ocfd_params* ps, int nsolve, const int* nblk_s, con
     L.tile_of = d_tile_of; L.err = h->d_lu_err; L.TJ = TJ; L.TK = TK;
     L.spin_limit = 4000000;  // x ~64 ns: a few hundred ms before a stuck wait gives up
     if (const char* sl = std::getenv("OCFD_LU_SPIN_LIMIT")) L.spin_limit = std::max(0LL, std::atoll(sl));
-    // version 5: each tile's edge words, (steps) x NV x (TJ + TK), all empty
+    // version 5: each tile's edge words, (steps) x NV x (TJ + TK)
     std::vector<long long> edge_off(first + 1, 0);
     for (int b = 0; b < nblk; b++)
       for (int q = tile_of[3 * b]; q < tile_of[3 * b] + tile_of[3 * b + 1] * tile_of[3 * b + 2]; q++)
@@ -1034,9 +1038,9 @@ static int create_impl(const ocfd_params* ps, int nsolve, const int* nblk_s, con
     L.edge = M.alloc<long long>((size_t)edge_off[first], e);
     if (e != cudaSuccess) { M.release(); return cuda_fail(nullptr, e, "lu edges"); }
     cudaMemcpy(d_edge_off, edge_off.data(), edge_off.size() * sizeof(long long), cudaMemcpyHostToDevice);
-    cudaMemset(L.edge, 0xFF, (size_t)edge_off[first] * sizeof(long long));
     L.edge_off = d_edge_off;
   }
+  reset_lu_edges(h);
   // ---- runner
   h->info.nvar = NV; h->info.time_method = p->time_method; h->info.viscous = p->if_viscous; h->info.turb = turb;
   h->info.smoothing = p->if_residual_smoothing;

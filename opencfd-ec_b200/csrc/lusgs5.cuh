@@ -36,8 +36,11 @@
 //
 // Cross-tile terms: an edge column's terms are stored to a buffer of this tile (edge_off), one
 // 8-byte word per value and step, and the consuming tile's warp E polls the words themselves: a
-// word holds the sentinel (all ones, a NaN no arithmetic produces) until its value is stored, and E
-// puts the sentinel back after reading it, so the buffer is ready for the next sweep.  No flag, no
+// word holds the sentinel until its value is stored, and E puts the sentinel back after reading it, so
+// the buffer is ready for the next sweep.  The sentinel is a signalling NaN: FP64 arithmetic carries a
+// quiet NaN's payload on (all ones, say, from a state filled with 0xFF), but the result of an operation
+// on a signalling NaN is a quiet one (IEEE 754, 6.2; checked on B200 for add, mul and fma), and every
+// term is the result of an operation.  No flag, no
 // fence: one store and one L2 read between tiles.  The wait is bounded (L.spin_limit); E then sets
 // the error flag and delivers zeros without waiting until the tile ends.  Deadlock freedom is that
 // of lusgs.cuh: tiles are handed out in topological order to resident CTAs.
@@ -63,7 +66,7 @@ namespace ocfd {
 // ns between a loader warp's requests: keeps bursts off the load path (wing-body sweep 1.37 -> 1.31 ms).
 // Flat from 300 to 400 (257x97x86 FP64 step 2.60 ms); 150 gives 2.64 ms, 700 gives 2.68 ms.
 constexpr int LU5_PACE = 300;
-constexpr long long LU5_EMPTY = -1LL;  // the sentinel of an edge word
+constexpr long long LU5_EMPTY = 0x7ff25ec0de5c0ffeLL;  // the sentinel of an edge word: a signalling NaN (quiet bit clear)
 
 // ---- division by a shared reciprocal -------------------------------------------------------
 // (rcp_rn, div_by and expo of double are in physics.cuh)
