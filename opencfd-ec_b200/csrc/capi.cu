@@ -1024,7 +1024,7 @@ static int create_impl(const ocfd_params* ps, int nsolve, const int* nblk_s, con
     L.tiles = d_tiles; L.rtiles = d_rtiles; L.utiles = d_utiles; L.ntiles = first; L.counter = d_counter; L.progress = d_progress;
     L.progress_up = d_progress_up; L.blkdone = d_blkdone;
     L.tile_of = d_tile_of; L.err = h->d_lu_err; L.TJ = TJ; L.TK = TK;
-    L.spin_limit = 4000000;  // x ~64 ns: a few hundred ms before a stuck wait gives up
+    L.spin_limit = 4000000;  // x ~64 ns: a few hundred ms before a stuck wait gives up (version 5: lu5_wait.h)
     if (const char* sl = std::getenv("OCFD_LU_SPIN_LIMIT")) L.spin_limit = std::max(0LL, std::atoll(sl));
     // version 5: each tile's edge words, (steps) x NV x (TJ + TK)
     std::vector<long long> edge_off(first + 1, 0);

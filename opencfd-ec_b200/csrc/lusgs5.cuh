@@ -40,10 +40,11 @@
 // the buffer is ready for the next sweep.  The sentinel is a signalling NaN: FP64 arithmetic carries a
 // quiet NaN's payload on (all ones, say, from a state filled with 0xFF), but the result of an operation
 // on a signalling NaN is a quiet one (IEEE 754, 6.2; checked on B200 for add, mul and fma), and every
-// term is the result of an operation.  No flag, no
-// fence: one store and one L2 read between tiles.  The wait is bounded (L.spin_limit); E then sets
-// the error flag and delivers zeros without waiting until the tile ends.  Deadlock freedom is that
-// of lusgs.cuh: tiles are handed out in topological order to resident CTAs.
+// term is the result of an operation.  No flag, no fence: one store and one L2 read between tiles.
+// The wait is bounded (L.spin_limit, lu5_wait.h); E then sets the error flag and delivers zeros without
+// waiting until the tile ends, and the tiles not yet begun are skipped, in this launch and in those
+// before the host has read the flag: a failure costs about two bounds, not one per tile.  Deadlock
+// freedom is that of lusgs.cuh: tiles are handed out in topological order to resident CTAs.
 //
 // Measured (B200, ms lower + upper sweep, the best of versions 3 and 4 -> this): config 2 (2.09 M
 // cells, 8 blocks) FP64 0.690 + 0.669 -> 0.491 + 0.493, mixed 0.623 + 0.664 -> 0.426 + 0.430; 64
@@ -59,6 +60,7 @@
 // warp bounds it), 64-column tiles (+60 %), face geometry and state loaded by the D and P warps
 // themselves into registers (+20 to 40 %).
 #pragma once
+#include "lu5_wait.h"
 #include "lusgs.cuh"
 
 namespace ocfd {
@@ -108,14 +110,20 @@ __device__ __forceinline__ bool mb_try(unsigned a, unsigned parity) {
 }
 __device__ __forceinline__ void mb_arrive(unsigned a) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(a) : "memory"); }
 // waits for the phase of the given parity; bounded (another role of the CTA always makes progress:
-// the bound only turns a defect into an error)
-__device__ __forceinline__ void mb_wait(unsigned a, unsigned parity, int* err) {
+// the bound only turns a defect into an error).  tries: the thread's bound, 0 once it has run out: its
+// later waits end after one try (the tile is lost, every access stays in its place)
+__device__ __forceinline__ void mb_wait(unsigned a, unsigned parity, int& tries, int* err) {
   for (int n = 0; !mb_try(a, parity);)
-    if (++n > 20000000) { atomicExch(err, 1); return; }
+    if (++n > tries) { tries = 0; atomicExch(err, 1); return; }
 }
 __device__ __forceinline__ long long ld_word(const long long* p) {
   long long v;
   asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ int ld_word32(const int* p) {
+  int v;
+  asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
 __device__ __forceinline__ void st_word(long long* p, long long v) { asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(v) : "memory"); }
@@ -176,7 +184,7 @@ __global__ void __launch_bounds__(7 * TC + 32, 1) k_lusgs_wave5(Arena<T> A, LuAr
   constexpr int AS5 = NV == 6 ? 2 : 0;  // the SA variable's own diagonal (FP64 form: value, reciprocal)
   extern __shared__ __align__(16) unsigned char s_dyn[];
   __shared__ __align__(8) unsigned long long s_bar[3 * SLOTS + 4];
-  __shared__ int s_tile;
+  __shared__ int s_tile, s_err;
   const long long tb = A.tot_box, tf = A.tot_face, tc = A.tot_cell;
   const int TJ = L.TJ, TK = L.TK;
   const int tid = threadIdx.x, role = tid / TC, c = tid % TC, lane = tid & 31;  // roles 0..2: D, 3, 4: P, 5, 6: L, 7: E
@@ -197,15 +205,20 @@ __global__ void __launch_bounds__(7 * TC + 32, 1) k_lusgs_wave5(Arena<T> A, LuAr
   // steps and row blocks this CTA has done (the same in every role): slot it % SLOTS, round
   // it / SLOTS; block buffer ib % 2, round ib / 2
   unsigned it = 0, ib = 0;
+  int tries = lu5_tries(L.spin_limit);
   for (;;) {
     __syncthreads();
-    if (tid == 0) s_tile = atomicAdd(&L.counter[UPPER ? 1 : 0], 1);
+    if (tid == 0) {
+      s_err = ld_word32(L.err);
+      s_tile = atomicAdd(&L.counter[UPPER ? 1 : 0], 1);
+    }
     __syncthreads();
     const int q = s_tile;
     if (q >= L.ntiles) {  // the last CTA to ask leaves the counter at 0 for the next sweep
       if (tid == 0 && q == L.ntiles + (int)gridDim.x - 1) L.counter[UPPER ? 1 : 0] = 0;
       break;
     }
+    if (s_err) continue;  // a wait has run out, in this launch or one before: the sweep is lost
     const LuTile tl = UPPER ? L.rtiles[q] : L.tiles[q];
     const BlkD& B = A.blk[tl.blk];
     const SolveP& s = A.sp[B.solve];
@@ -334,7 +347,7 @@ __global__ void __launch_bounds__(7 * TC + 32, 1) k_lusgs_wave5(Arena<T> A, LuAr
       };
       T F[2][NV];
       Cell x[2];
-      mb_wait(fullP + 8 * (it % SLOTS), (it / SLOTS) & 1, L.err);
+      mb_wait(fullP + 8 * (it % SLOTS), (it / SLOTS) & 1, tries, L.err);
       take(x[0], slot_of(it), row_of(0));
       if (old_flux(x[0], F[0], false)) old_flux(x[0], F[0], true);
       for (int t0 = 0; t0 < nsteps; t0 += 2) {
@@ -353,7 +366,7 @@ __global__ void __launch_bounds__(7 * TC + 32, 1) k_lusgs_wave5(Arena<T> A, LuAr
             const unsigned ea = fullE + 8 * (n % SLOTS), ep = (n / SLOTS) & 1;
             const unsigned pa = t + 1 < nsteps ? fullP + 8 * ((n + 1) % SLOTS) : ea, pp = t + 1 < nsteps ? ((n + 1) / SLOTS) & 1 : ep;
             const bool e0 = mb_try(ea, ep), p0 = mb_try(pa, pp);
-            if (!(e0 && p0)) { mb_wait(ea, ep, L.err); mb_wait(pa, pp, L.err); }
+            if (!(e0 && p0)) { mb_wait(ea, ep, tries, L.err); mb_wait(pa, pp, tries, L.err); }
           }
           cta_bar_id<1, 3 * TC>();  // the terms of step t - 1 are in slot t
           double xs[NV];
@@ -414,7 +427,7 @@ __global__ void __launch_bounds__(7 * TC + 32, 1) k_lusgs_wave5(Arena<T> A, LuAr
       for (int t = role - 3; t < nsteps; t += 2) {  // even or odd steps of the tile
         const unsigned n = it + t, rb = ib + t / WB;
         unsigned char* const sl = slot_of(n);
-        if (t % WB < 2) mb_wait(fullR + 8 * (rb & 1), (rb >> 1) & 1, L.err);  // this warp's first step of the block
+        if (t % WB < 2) mb_wait(fullR + 8 * (rb & 1), (rb >> 1) & 1, tries, L.err);  // this warp's first step of the block
         const int row = row_of(t);
         const unsigned char* const r8 = s_dyn + row * PB + c * 8;
         const unsigned char* const rt = s_dyn + row * PT + c * (int)sizeof(T);
@@ -456,7 +469,7 @@ __global__ void __launch_bounds__(7 * TC + 32, 1) k_lusgs_wave5(Arena<T> A, LuAr
         }
         double ra = rcp_rn(al), ras = NV == 6 ? rcp_rn(als) : 0.0;
         if (bad_den(al) || (NV == 6 && bad_den(als))) { ra = 1.0 / al; ras = 1.0 / als; }
-        mb_wait(empty0 + 8 * (n % SLOTS), (n / SLOTS + 1) & 1, L.err);  // the slot's last readers are done
+        mb_wait(empty0 + 8 * (n % SLOTS), (n / SLOTS + 1) & 1, tries, L.err);  // the slot's last readers are done
         if constexpr (NA == 1) {
           reinterpret_cast<double*>(sl + SM::AL)[c] = ra;
         } else {
@@ -503,7 +516,7 @@ __global__ void __launch_bounds__(7 * TC + 32, 1) k_lusgs_wave5(Arena<T> A, LuAr
         const unsigned gb = ib + wb;
         const int row = (int)(gb & 1) * WB + iw;
         if (wb >= 2) {  // block wb - 2 is done: its DU to memory, then its rows are free
-          mb_wait(emptyR + 8 * (gb & 1), ((gb - 2) >> 1) & 1, L.err);
+          mb_wait(emptyR + 8 * (gb & 1), ((gb - 2) >> 1) & 1, tries, L.err);
           const int t = (wb - 2) * WB + iw;
 #pragma unroll
           for (int r = 0; r < NR; r++) {
@@ -577,7 +590,8 @@ __global__ void __launch_bounds__(7 * TC + 32, 1) k_lusgs_wave5(Arena<T> A, LuAr
           }
         }
       }
-      long long spins = 0;
+      const int rounds = lu5_rounds(L.spin_limit);
+      int spins = 0;
       bool gave_up = false;
       int t = 0;
       while (t < nsteps) {
@@ -601,7 +615,7 @@ __global__ void __launch_bounds__(7 * TC + 32, 1) k_lusgs_wave5(Arena<T> A, LuAr
           ready += all ? 1 : 0;
         }
         if (ready == 0) {
-          if (++spins > L.spin_limit) {
+          if (++spins > rounds) {
             gave_up = true;
             if (lane == 0) atomicExch(L.err, 1);
           }
@@ -613,7 +627,7 @@ __global__ void __launch_bounds__(7 * TC + 32, 1) k_lusgs_wave5(Arena<T> A, LuAr
           if (g >= ready) break;
           const unsigned n = it + t + g;
           double* const acc = reinterpret_cast<double*>(slot_of(n) + SM::ACC);
-          mb_wait(empty0 + 8 * (n % SLOTS), (n / SLOTS + 1) & 1, L.err);
+          mb_wait(empty0 + 8 * (n % SLOTS), (n / SLOTS + 1) & 1, tries, L.err);
 #pragma unroll
           for (int e = 0; e < EPL; e++) {
             const int il = t + g - lo[e];
@@ -631,6 +645,7 @@ __global__ void __launch_bounds__(7 * TC + 32, 1) k_lusgs_wave5(Arena<T> A, LuAr
     it += nsteps;
     ib += nblk;
   }
+  asm volatile("cp.async.wait_all;" ::: "memory");  // none is in flight unless a wait ran out
 }
 
 template <class T, int NV, int TC>
