@@ -345,6 +345,12 @@ int ocfd_lu_kernel_version(const ocfd_handle* h);
  * selects it; same results, slower than version 5 and than the two launches of version 4).  ocfd_profile then reports the joint time as the lower
  * sweep's and 0 for the upper. */
 int ocfd_lu_one_launch(const ocfd_handle* h);
+/* Bound of each wait between tiles of the handle's LU-SGS sweeps from the next step on, in polls of
+ * about 64 ns (created with 4,000,000 or OCFD_LU_SPIN_LIMIT).  A wait that runs out makes the next
+ * ocfd_residual, ocfd_residual_all or ocfd_residual_static return OCFD_ERR_TIMEOUT; the state is lost
+ * (set it again, or ocfd_init_flow), the handle stays usable.  Drops the captured step graph, which the
+ * next ocfd_advance captures again. */
+int ocfd_set_lu_wait_limit(ocfd_handle* h, long long limit);
 
 #ifdef __cplusplus
 }

@@ -438,6 +438,14 @@ static void autotune_lu(ocfd_handle* h, const std::vector<std::pair<int, int>>& 
 
 extern "C" int ocfd_lu_tile_width(const ocfd_handle* h) { return h ? h->lu_tc : 0; }
 extern "C" int ocfd_lu_kernel_version(const ocfd_handle* h) { return h ? h->info.lu_version : 0; }
+extern "C" int ocfd_set_lu_wait_limit(ocfd_handle* h, long long limit) {
+  if (!h || limit < 0) return OCFD_ERR_ARG;
+  cudaError_t e = cudaStreamSynchronize(h->st);
+  if (e != cudaSuccess) return cuda_fail(h, e, "set_lu_wait_limit");
+  for (LuArgs& L : h->lu_var) L.spin_limit = limit;
+  select_lu(h, h->lu_tc == 64 ? 1 : 0, h->info.lu_fused ? 6 : h->info.lu_version);
+  return h->run ? OCFD_OK : fail(h, OCFD_ERR_UNSUPPORTED, "set_lu_wait_limit");
+}
 extern "C" int ocfd_lu_one_launch(const ocfd_handle* h) {
   return h && !h->info.lu_planes && h->info.lu_version == 4 && h->info.lu_fused ? 1 : 0;
 }
@@ -1642,8 +1650,8 @@ static int residual_impl(ocfd_handle* h, double* rmax, double* rrms, int nout) {
       rmax[7 * q + m] = m < h->nvar ? out[14 * q + m] : 0.0;
       rrms[7 * q + m] = m < h->nvar ? std::sqrt(out[14 * q + 7 + m] / (double)h->ncell_s[q]) : 0.0;
     }
-  if (lu_err) {
-    cudaMemset(h->d_lu_err, 0, 4);
+  if (lu_err) {  // on the handle's stream: the next sweep must not see the old flag, it would skip its tiles
+    cudaMemsetAsync(h->d_lu_err, 0, 4, h->st);
     reset_lu_edges(h);
     return fail(h, OCFD_ERR_TIMEOUT, "LU-SGS wavefront: a bounded wait between tiles timed out");
   }

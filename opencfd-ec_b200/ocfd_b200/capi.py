@@ -75,6 +75,7 @@ def lib():
         L.ocfd_lu_tile_width.argtypes = [vp]
         L.ocfd_lu_kernel_version.argtypes = [vp]
         L.ocfd_lu_one_launch.argtypes = [vp]
+        L.ocfd_set_lu_wait_limit.argtypes = [vp, ctypes.c_longlong]
         _lib = L
     return _lib
 
@@ -238,6 +239,10 @@ class Solver:
     def lu_one_launch(self):
         """True when both LU-SGS sweeps run as one launch (profile() then reports them as the lower one)."""
         return bool(lib().ocfd_lu_one_launch(self.h))
+
+    def set_lu_wait_limit(self, limit):
+        """Bound of each wait between tiles of the LU-SGS sweeps, in polls of about 64 ns."""
+        self._check(lib().ocfd_set_lu_wait_limit(self.h, int(limit)), "set_lu_wait_limit")
 
     def synchronize(self):
         self._check(lib().ocfd_synchronize(self.h), "synchronize")
