@@ -378,7 +378,6 @@ static void reset_work(ocfd_handle* h) {
   reset_mu(h);
 }
 
-// version-5 record layout for the handle's precision and NVAR
 // (re)builds the runner for LU-SGS tile table v (0: TC = 32, 1: TC = 64) and wavefront kernel
 // version ver (2 to 5); drops a captured graph
 static void select_lu(ocfd_handle* h, int v, int ver) {
@@ -434,6 +433,34 @@ static void autotune_lu(ocfd_handle* h, const std::vector<std::pair<int, int>>& 
   for (int q = 0; q < 6; q++) cudaEventDestroy(ev[q]);
   reset_work(h);
   select_lu(h, bestv.first, bestv.second);
+}
+
+// LU-SGS kernel of a new handle: (tile table, version) candidates, timed against each other where there
+// are several.  Version 5 on 32-column tiles, the fastest form on every configuration (config 2: 0.49 ms
+// a sweep against 0.69 of the best of versions 3 and 4, its 64-column form 0.82; see lusgs5.cuh).
+// OCFD_LU_TC fixes the tile width, OCFD_LU_V3 / V4 / V5 the version (OCFD_LU_V2 both); versions 3 and 4
+// are timed against each other where the switches leave a choice, and OCFD_NO_AUTOTUNE takes the first
+// of them.  OCFD_LU_ONE_LAUNCH puts version 4's one-launch form (6: k_lusgs_wave4_ul) in its place.
+// Steps that do not sweep (explicit schemes) or not in tiles (OCFD_LUSGS_PLANES) leave version 4, which
+// keeps no edge words (18 to 27 B a cell).
+static std::vector<std::pair<int, int>> lu_candidates(int time_method) {
+  auto on = [](const char* name) { return std::getenv(name) != nullptr; };
+  const char* tc = std::getenv("OCFD_LU_TC");
+  const int force_tc = !tc ? 0 : (std::atoi(tc) == 64 ? 64 : 32);
+  const int force_ver = on("OCFD_LU_V3") ? 3 : (on("OCFD_LU_V4") ? 4 : (on("OCFD_LU_V5") ? 5 : 0));
+  const bool one = on("OCFD_LU_ONE_LAUNCH"), no_sweep = time_method == 1 || time_method == 3 || on("OCFD_LUSGS_PLANES");
+  if (on("OCFD_LU_V2")) return {{1, 2}};
+  if (force_ver == 5) return {{force_tc == 64 ? 1 : 0, 5}};
+  if (!force_ver && force_tc != 64 && !one && !on("OCFD_NO_AUTOTUNE")) return {{0, no_sweep ? 4 : 5}};
+  std::vector<std::pair<int, int>> cand;
+  for (int v = 0; v < 2; v++) {
+    if (force_tc && (force_tc == 64) != (v == 1)) continue;
+    for (int ver : {4, 3}) {
+      if (force_ver && ver != force_ver) continue;
+      cand.push_back({v, ver == 4 && one ? 6 : ver});
+    }
+  }
+  return cand;
 }
 
 extern "C" int ocfd_lu_tile_width(const ocfd_handle* h) { return h ? h->lu_tc : 0; }
@@ -960,12 +987,8 @@ static int create_impl(const ocfd_params* ps, int nsolve, const int* nblk_s, con
   }
   if ((e = cudaStreamSynchronize(h->st)) != cudaSuccess) { M.release(); return cuda_fail(nullptr, e, "geometry sync"); }
   // ---- LU-SGS wavefront tiles: TJ x TK = TC columns per CTA, ordered by J+K.  Tables are built
-  //      for both tile widths (TC = 32 and 64); the faster one on this case is picked at the end
-  //      of creation (OCFD_LU_TC=32|64 fixes it; the one-thread-per-column form uses TC = 64)
-  const int lu_v2 = std::getenv("OCFD_LU_V2") ? 1 : 0;
-  int lu_force = 0;
-  if (const char* e2 = std::getenv("OCFD_LU_TC")) lu_force = std::atoi(e2) == 64 ? 64 : 32;
-  if (lu_v2) lu_force = 64;
+  //      for both tile widths (TC = 32 and 64); lu_candidates says which one the sweeps use
+  const std::vector<std::pair<int, int>> lu_cand = lu_candidates(p->time_method);
   h->d_lu_err = M.alloc<int>(1, e);
   int* d_counter = M.alloc<int>(2, e);
   for (int v = 0; v < 2; v++) {
@@ -1034,13 +1057,13 @@ static int create_impl(const ocfd_params* ps, int nsolve, const int* nblk_s, con
     L.tile_of = d_tile_of; L.err = h->d_lu_err; L.TJ = TJ; L.TK = TK;
     L.spin_limit = 4000000;  // x ~64 ns: a few hundred ms before a stuck wait gives up (version 5: lu5_wait.h)
     if (const char* sl = std::getenv("OCFD_LU_SPIN_LIMIT")) L.spin_limit = std::max(0LL, std::atoll(sl));
+    if (lu_cand[0] != std::make_pair(v, 5)) continue;
     // version 5: each tile's edge words, (steps) x NV x (TJ + TK)
     std::vector<long long> edge_off(first + 1, 0);
     for (int b = 0; b < nblk; b++)
       for (int q = tile_of[3 * b]; q < tile_of[3 * b] + tile_of[3 * b + 1] * tile_of[3 * b + 2]; q++)
         edge_off[q + 1] = (long long)(h->blk[b].nx - 1 + TJ + TK - 2) * NV * (TJ + TK);
     for (int q = 0; q < first; q++) edge_off[q + 1] += edge_off[q];
-    if (v == 1 && !std::getenv("OCFD_LU_V5")) continue;  // 64-column tiles run version 5 only when it is asked for
     h->lu_edge_words[v] = edge_off[first];
     long long* d_edge_off = M.alloc<long long>(edge_off.size(), e);
     L.edge = M.alloc<long long>((size_t)edge_off[first], e);
@@ -1108,26 +1131,6 @@ static int create_impl(const ocfd_params* ps, int nsolve, const int* nblk_s, con
   }
   if (h->prec == OCFD_PREC_MIXED) fill_arena<float>(h, h->A32, h->d_Mf, h->d_volf, h->d_dtmf, h->d_dwf);
   else fill_arena<double>(h, h->A64, h->d_Md, h->d_vold, h->d_dtmd, h->d_dwd);
-  // LU-SGS kernel: version 5 on 32-column tiles, the fastest form on every configuration (config 2:
-  // 0.49 ms a sweep against 0.69 of the best of versions 3 and 4, its 64-column form 0.82; see
-  // lusgs5.cuh).  OCFD_LU_TC fixes the tile width, OCFD_LU_V3 / V4 / V5 the version (OCFD_LU_V2
-  // both); versions 3 and 4 are timed against each other where the switches leave a choice, and
-  // OCFD_NO_AUTOTUNE takes the first of them.  OCFD_LU_ONE_LAUNCH puts version 4's one-launch form
-  // (6: k_lusgs_wave4_ul) in its place
-  const int lu_ver_force = lu_v2 ? 2 : (std::getenv("OCFD_LU_V3") ? 3 : (std::getenv("OCFD_LU_V4") ? 4 : (std::getenv("OCFD_LU_V5") ? 5 : 0)));
-  const bool lu_one = std::getenv("OCFD_LU_ONE_LAUNCH") != nullptr;
-  std::vector<std::pair<int, int>> lu_cand;
-  if (lu_ver_force == 2) lu_cand.push_back({1, 2});
-  else if (lu_ver_force == 5) lu_cand.push_back({lu_force == 64 ? 1 : 0, 5});
-  else if (!lu_ver_force && lu_force != 64 && !lu_one && !std::getenv("OCFD_NO_AUTOTUNE")) lu_cand.push_back({0, 5});
-  else
-    for (int v = 0; v < 2; v++) {
-      if (lu_force && (lu_force == 64) != (v == 1)) continue;
-      for (int ver : {4, 3}) {
-        if (lu_ver_force && ver != lu_ver_force) continue;
-        lu_cand.push_back({v, ver == 4 && lu_one ? 6 : ver});
-      }
-    }
   select_lu(h, lu_cand[0].first, lu_cand[0].second);
   if (!h->run) { M.release(); return OCFD_ERR_UNSUPPORTED; }
   if (lu_cand.size() > 1 && !h->info.lu_planes && !std::getenv("OCFD_NO_AUTOTUNE")) {
@@ -1388,12 +1391,12 @@ extern "C" long long ocfd_footprint(const ocfd_params* p, int nblk, const int* n
   if (tm == 3) bytes += ts * (2 * tb + tf);
   if (p->precision == OCFD_PREC_MIXED) bytes += 4 * (M_COUNT * tf + 3 * tc);
   bytes += NV * maxbox * 8;                                                       // state staging
-  // LU-SGS version 5: the edge words of the 32-column tiles, (TJ + TK) NV per step and tile
-  const int v5n = std::getenv("OCFD_LU_V5") ? 2 : 1;
-  int min_nzm = 1 << 30;
-  for (int b = 0; b < nblk; b++) min_nzm = std::min(min_nzm, nijk[3 * b + 2] - 1);
-  for (int v = 0; v < v5n; v++) {
-    const int tcv = v == 0 ? 32 : 64, TK = min_nzm <= 2 ? 2 : (min_nzm <= 4 || v == 0 ? 4 : 8), TJ = tcv / TK;
+  // LU-SGS version 5: the edge words, (TJ + TK) NV per step and tile
+  const std::pair<int, int> lu = lu_candidates(p->time_method)[0];
+  if (lu.second == 5) {
+    int min_nzm = 1 << 30;
+    for (int b = 0; b < nblk; b++) min_nzm = std::min(min_nzm, nijk[3 * b + 2] - 1);
+    const int v = lu.first, tcv = v == 0 ? 32 : 64, TK = min_nzm <= 2 ? 2 : (min_nzm <= 4 || v == 0 ? 4 : 8), TJ = tcv / TK;
     for (int b = 0; b < nblk; b++) {
       const long long nJ = (nijk[3 * b + 1] - 1 + TJ - 1) / TJ, nK = (nijk[3 * b + 2] - 1 + TK - 1) / TK;
       bytes += 8 * NV * (TJ + TK) * nJ * nK * (nijk[3 * b] - 1 + TJ + TK - 2);
