@@ -22,7 +22,8 @@ EXPORTED = [
     "ocfd_limiter_status", "ocfd_array_shape", "ocfd_get_array", "ocfd_version", "ocfd_compute_residual",
     "ocfd_stream", "ocfd_profile", "ocfd_launches_per_step", "ocfd_create_batch", "ocfd_nsolve", "ocfd_reset_solve",
     "ocfd_residual_all", "ocfd_forces_all", "ocfd_footprint", "ocfd_synchronize", "ocfd_residual_static",
-    "ocfd_lu_tile_width", "ocfd_lu_kernel_version", "ocfd_lu_one_launch", "ocfd_create_part", "ocfd_part_blocks", "ocfd_part_plan",
+    "ocfd_lu_tile_width", "ocfd_lu_kernel_version", "ocfd_lu_one_launch", "ocfd_set_lu_wait_limit", "ocfd_create_part",
+    "ocfd_part_blocks", "ocfd_part_plan",
 ]
 
 
