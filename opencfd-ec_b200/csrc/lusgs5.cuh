@@ -209,8 +209,9 @@ __global__ void __launch_bounds__(7 * TC + 32, 1) k_lusgs_wave5(Arena<T> A, LuAr
   for (;;) {
     __syncthreads();
     if (tid == 0) {
-      s_err = ld_word32(L.err);
-      s_tile = atomicAdd(&L.counter[UPPER ? 1 : 0], 1);
+      const int e = ld_word32(L.err), n = atomicAdd(&L.counter[UPPER ? 1 : 0], 1);  // both in flight at once
+      s_err = e;
+      s_tile = n;
     }
     __syncthreads();
     const int q = s_tile;
@@ -565,6 +566,7 @@ __global__ void __launch_bounds__(7 * TC + 32, 1) k_lusgs_wave5(Arena<T> A, LuAr
         }
         cp_arrive(fullR + 8 * (gb & 1));
       }
+      asm volatile("cp.async.wait_all;" ::: "memory");  // none is in flight unless a wait ran out
     } else {
       // ------------------------------------------------------------------ terms from the upstream tiles
       constexpr int EPL = (NV * (TC / 2 + 2) + 31) / 32, W = EPL > 4 ? 2 : 4;  // words per lane and step; steps polled at once
@@ -645,7 +647,6 @@ __global__ void __launch_bounds__(7 * TC + 32, 1) k_lusgs_wave5(Arena<T> A, LuAr
     it += nsteps;
     ib += nblk;
   }
-  asm volatile("cp.async.wait_all;" ::: "memory");  // none is in flight unless a wait ran out
 }
 
 template <class T, int NV, int TC>
