@@ -332,8 +332,9 @@ int ocfd_profile(ocfd_handle* h, int nsteps, double* phase_ms);
 int ocfd_launches_per_step(ocfd_handle* h);
 /* Columns per CTA tile (32 or 64) of the LU-SGS wavefront sweeps, and the wavefront kernel version
  * in use: 5 (the default, on 32-column tiles: every term evaluated once by the producing cell, one
- * task per warp); 4: inputs staged by 32-byte sector, 3: by element; 2: one thread per column.  Every
- * version gives the same results.  OCFD_LU_TC=32|64 fixes the width, OCFD_LU_V3 / V4 / V5=1 the
+ * task per warp); 4: inputs staged by 32-byte sector, 3: by element; 2: one thread per column.  Handles
+ * whose steps do not sweep (time_method 1 and 3) keep version 4, which ocfd_compute_residual runs when
+ * it is asked for the sweeps.  Every version gives the same results.  OCFD_LU_TC=32|64 fixes the width, OCFD_LU_V3 / V4 / V5=1 the
  * version; with versions 3 and 4 ocfd_create times what the switches leave open on the new case (a
  * few steps from freestream, before the state is initialised) and keeps the fastest, unless
  * OCFD_NO_AUTOTUNE=1, which takes version 4 (64 columns if fixed, else 32) where no version is

@@ -442,7 +442,7 @@ static void autotune_lu(ocfd_handle* h, const std::vector<std::pair<int, int>>& 
 // are timed against each other where the switches leave a choice, and OCFD_NO_AUTOTUNE takes the first
 // of them.  OCFD_LU_ONE_LAUNCH puts version 4's one-launch form (6: k_lusgs_wave4_ul) in its place.
 // Steps that do not sweep (explicit schemes) or not in tiles (OCFD_LUSGS_PLANES) leave version 4, which
-// keeps no edge words (18 to 27 B a cell).
+// keeps no edge words (8 NV (TJ + TK) / 32 B a cell: 15 to 32).
 static std::vector<std::pair<int, int>> lu_candidates(int time_method) {
   auto on = [](const char* name) { return std::getenv(name) != nullptr; };
   const char* tc = std::getenv("OCFD_LU_TC");
@@ -1948,7 +1948,8 @@ __global__ void k_gather_array(GatherD d, double* out) {
 
 // copies the array in the requested Fortran bounds, interleaved on the device into the state's
 // staging area and read back in one transfer (a host loop over the values took most of the call: state in,
-// residual, 131,072 x 5 FP32 values out 2.13 -> 1.30 ms)
+// residual, 131,072 x 5 FP32 values out 2.13 -> 1.30 ms where the caller's array has been touched before;
+// on pages that have not, their faults and the pageable copy are most of what is left)
 extern "C" int ocfd_get_array(ocfd_handle* h, int b, const char* name, double* out) {
   if (!h || !name || !out || b < 0 || b >= h->nblk) return OCFD_ERR_ARG;
   ArrDesc d;

@@ -14,8 +14,10 @@
 //   * the quotients by one denominator share its reciprocal: r = RN(1/b), q = RN(x r),
 //     q' = RN(q + r RN(x - b q)), the FMA division of Markstein (IBM J. Res. Dev. 34, 1990; Cornea,
 //     Harrison and Tang, "Scientific Computing on Itanium", 2002), correctly rounded, hence the
-//     bits of x / b, without a branch.  Operands near the limits of the format, infinities and NaN
-//     take the plain division.
+//     bits of x / b, without a branch.  Large operands, small denominators, infinities and NaN take
+//     the plain division (bad_den, bad_num).  Small numerators do not: -0 / b gives +0, and a
+//     numerator whose remainder x - b q is subnormal (below about 2^-969 in FP64, 2^-103 in FP32)
+//     can give a quotient one unit off.
 //
 // Warps of a CTA (TC columns per tile, TC = 32 or 64; RW = TC / 32 warps per group):
 //   L (2 RW)    loads every input plane of the tile in blocks of WB steps, two blocks deep: a request
@@ -50,10 +52,10 @@
 // cells, 8 blocks) FP64 0.690 + 0.669 -> 0.491 + 0.493, mixed 0.623 + 0.664 -> 0.426 + 0.430; 64
 // airfoils mixed 0.742 + 0.704 -> 0.459 + 0.435; wing-body (7.8 M cells, SST) mixed 1.62 + 1.65 -> 1.30
 // + 1.29; one 129 x 33 airfoil FP64 0.194 -> 0.110 a sweep, the 129 x 65 x 17 channel 0.33 -> 0.16.  A
-// step takes about 1,300 cycles: a D warp's ~320 instructions at four to five cycles each (a chain of
+// step takes about 1,400 cycles: a D warp's ~320 instructions at four to five cycles each (a chain of
 // dependent FP64 operations and shared-memory reads), beside the SM's load path at about half of its
-// rate (ncu on the channel, a step of a tile: 1,566 warp instructions of all roles, 666 wavefronts, of
-// which 263 shared-memory loads, 198 of L's copies and 69 stores).  Tried on top and slower: step
+// rate (ncu on the channel, a step of a tile: 1,558 warp instructions of all roles, 666 wavefronts, of
+// which 263 shared-memory loads, 198 of L's copies and 70 stores).  Tried on top and slower: step
 // counters with acquire loads in place of the mbarriers (+3 %), DU shared between the D warps by
 // variables with a second barrier (FP64 +15 %, mixed even), next step's mbarriers probed a step ahead
 // (even), two CTAs per SM at 168 registers with one P and one L warp (config 2 FP64 +90 %: the single L
@@ -87,7 +89,8 @@ __device__ __forceinline__ bool bad_num(unsigned e, float) { return e > 0x5f0000
 // The expressions of the flux difference.  FP64 rounds every operation, as the reference; the mixed
 // form contracts them exactly as versions 3 and 4 compile (which product of a sum enters the FMA
 // unrounded was found by comparing bits on random states; the compiler may choose otherwise in other
-// code), so that every version of the sweep gives the same bits.
+// code), so that every version of the sweep gives the same bits (halving the face area and radius first
+// is exact but where an FP32 product is subnormal).
 __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }

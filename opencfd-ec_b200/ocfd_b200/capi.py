@@ -234,7 +234,8 @@ class Solver:
         return int(lib().ocfd_lu_tile_width(self.h))
 
     def lu_kernel_version(self):
-        """LU-SGS wavefront kernel version in use (5 unless a switch selects another)."""
+        """LU-SGS wavefront kernel version in use (5 unless a switch selects another; 4 where the
+        steps do not sweep)."""
         return int(lib().ocfd_lu_kernel_version(self.h))
 
     def lu_one_launch(self):
