@@ -129,6 +129,7 @@ struct ocfd_handle {
   void *d_Res = nullptr, *d_dt = nullptr, *d_Lc = nullptr, *d_Lv = nullptr, *d_Fi = nullptr, *d_Fv = nullptr, *d_Ft = nullptr;
   int* d_flags = nullptr;
   double *d_norm_part = nullptr, *d_norm_out = nullptr, *d_force_part = nullptr, *d_stage = nullptr;
+  std::mutex stage_mu;         // d_stage: one set_state, get_state or get_array at a time, and no capture beside them
   unsigned long long* d_nan = nullptr;
   double* h_pin = nullptr;  // pinned read-back area of the monitors: norms, NaN location, wait flag, force partials
   long long max_box_b = 0;
@@ -1437,6 +1438,7 @@ extern "C" int ocfd_set_state(ocfd_handle* h, int b, const double* U) {
   if (!h || !U || b < 0 || b >= h->nblk) return OCFD_ERR_ARG;
   const BlkD& B = h->blk[b];
   long long box = (long long)B.NX * B.NY * B.NZ;
+  std::lock_guard<std::mutex> lk(h->stage_mu);
   cudaError_t e = cudaMemcpyAsync(h->d_stage, U, (size_t)h->nvar * box * 8, cudaMemcpyHostToDevice, h->st);
   if (e != cudaSuccess) return cuda_fail(h, e, "set_state");
   h->run->scatter_state(h->st, b, h->d_stage, box);
@@ -1449,6 +1451,7 @@ extern "C" int ocfd_get_state(ocfd_handle* h, int b, double* U) {
   if (!h || !U || b < 0 || b >= h->nblk) return OCFD_ERR_ARG;
   const BlkD& B = h->blk[b];
   long long box = (long long)B.NX * B.NY * B.NZ;
+  std::lock_guard<std::mutex> lk(h->stage_mu);
   h->run->gather_state(h->st, b, h->d_stage, box);
   cudaError_t e = cudaMemcpyAsync(U, h->d_stage, (size_t)h->nvar * box * 8, cudaMemcpyDeviceToHost, h->st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->st);
@@ -1521,6 +1524,7 @@ extern "C" int ocfd_init_flow(ocfd_handle* h) {
 static int ensure_graph(ocfd_handle* h) {
   if (h->gexec) return OCFD_OK;
   if (std::getenv("OCFD_NO_GRAPH") || h->part) return OCFD_OK;  // a sharded step calls back to the host
+  std::lock_guard<std::mutex> lk(h->stage_mu);
   cudaError_t e = cudaStreamBeginCapture(h->st, cudaStreamCaptureModeThreadLocal);
   if (e != cudaSuccess) return cuda_fail(h, e, "capture begin");
   h->run->step(h->st);
@@ -1964,6 +1968,7 @@ extern "C" int ocfd_get_array(ocfd_handle* h, int b, const char* name, double* o
   g.w0 = (unsigned)(d.hi[0] - d.lo[0] + 1);
   g.w1 = (unsigned)(d.hi[1] - d.lo[1] + 1);
   g.cells = (long long)g.w0 * g.w1 * (d.hi[2] - d.lo[2] + 1);
+  std::lock_guard<std::mutex> lk(h->stage_mu);
   k_gather_array<<<(int)std::min<long long>((g.cells + 255) / 256, 148 * 16), 256, 0, h->st>>>(g, h->d_stage);
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaMemcpyAsync(out, h->d_stage, sizeof(double) * g.nv * g.cells, cudaMemcpyDeviceToHost, h->st);
