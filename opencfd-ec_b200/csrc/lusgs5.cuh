@@ -521,6 +521,9 @@ __global__ void __launch_bounds__(7 * TC + 32, 1) k_lusgs_wave5(Arena<T> A, LuAr
         const int row = (int)(gb & 1) * WB + iw;
         if (wb >= 2) {  // block wb - 2 is done: its DU to memory, then its rows are free
           mb_wait(emptyR + 8 * (gb & 1), ((gb - 2) >> 1) & 1, tries, L.err);
+          // its copies have landed long since, unless a wait ran out: none may be in flight at the kernel's end
+          // (cp.async.wait_all there instead costs 1 us a sweep, even behind a branch that is never taken)
+          mb_wait(fullR + 8 * (gb & 1), ((gb - 2) >> 1) & 1, tries, L.err);
           const int t = (wb - 2) * WB + iw;
 #pragma unroll
           for (int r = 0; r < NR; r++) {
@@ -569,7 +572,6 @@ __global__ void __launch_bounds__(7 * TC + 32, 1) k_lusgs_wave5(Arena<T> A, LuAr
         }
         cp_arrive(fullR + 8 * (gb & 1));
       }
-      asm volatile("cp.async.wait_all;" ::: "memory");  // none is in flight unless a wait ran out
     } else {
       // ------------------------------------------------------------------ terms from the upstream tiles
       constexpr int EPL = (NV * (TC / 2 + 2) + 31) / 32, W = EPL > 4 ? 2 : 4;  // words per lane and step; steps polled at once
